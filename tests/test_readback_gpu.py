@@ -1,0 +1,88 @@
+"""Device-to-host copies of diagnostics and the kept workspace: every byte arrives at the sizes where the
+copy changes its path (direct, one lane, several lanes, ragged last parts), from several threads at once;
+single-step calls give the same run before and after they switch to a captured step."""
+import threading
+
+import numpy as np
+import pytest
+
+import zpic_b200 as zb
+
+pytestmark = pytest.mark.gpu
+
+
+def _sim(ntiles, nx):
+    dx = 0.1
+    return zb.Simulation(ntiles, nx, (ntiles[0] * nx[0] * dx, ntiles[1] * nx[1] * dx), 0.05)
+
+
+# bytes of one grid: 364 * 12 = 4,368 per 16x16 tile; 64 KiB lies between 15 and 16 tiles, 512 KiB (a chunk)
+# between 120 and 121, 1 MiB at 240.05, 2 MiB at 480.1, 4 MiB at 960.2
+@pytest.mark.parametrize('ntiles', [(1, 1), (5, 3), (4, 4), (12, 10), (11, 11), (16, 15), (241, 1), (30, 16), (37, 13),
+                                    (31, 31), (64, 61)])
+def test_grid_round_trip(ntiles):
+    s = _sim(ntiles, (16, 16))
+    a = np.random.default_rng(ntiles[0]).random((ntiles[0] * ntiles[1], s.tile_vol, 3), np.float32)
+    s.set_grid('E', a)
+    s.set_grid('B', -a)
+    assert np.array_equal(s.grid('E'), a)
+    assert np.array_equal(s.grid('B'), -a)
+    # dense components use the kept workspace
+    d = a[:, :361].reshape(ntiles[1], ntiles[0], 19, 19, 3)[:, :, 1:17, 1:17].transpose(0, 2, 1, 3, 4)
+    for k in range(3):
+        assert np.array_equal(s.grid_gather('E', k), d.reshape(ntiles[1] * 16, ntiles[0] * 16, 3)[..., k])
+
+
+def test_pinned_destination():
+    import ctypes
+    import torch
+    s = _sim((16, 16), (16, 16))
+    a = np.random.default_rng(1).random((256, s.tile_vol, 3), np.float32)
+    s.set_grid('E', a)
+    t = torch.zeros(a.shape, dtype=torch.float32).pin_memory()
+    zb._check(zb.lib().zpic_b200_grid_get(s.h, 0, ctypes.cast(t.data_ptr(), ctypes.POINTER(ctypes.c_float))))
+    assert np.array_equal(t.numpy(), a)
+
+
+def test_threads_share_the_lanes():
+    sims, data, bad = [], [], []
+    for k in range(4):
+        s = _sim((30, 20), (16, 16))
+        a = np.random.default_rng(k).random((600, s.tile_vol, 3), np.float32)
+        s.set_grid('E', a)
+        sims.append(s)
+        data.append(a)
+
+    def work(k):
+        for _ in range(5):
+            if not np.array_equal(sims[k].grid('E'), data[k]):
+                bad.append(k)
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not bad
+    # the lanes are given back with the last simulation and made again
+    for s in sims:
+        s.close()
+    s = _sim((30, 20), (16, 16))
+    s.set_grid('E', data[0])
+    assert np.array_equal(s.grid('E'), data[0])
+
+
+def test_single_steps_equal_a_run():
+    """One species, one CTA per tile: the fixed-point tile current does not depend on the order of its sums,
+    so every field value is the same bit for bit however the steps are asked for."""
+    runs = []
+    for parts in ([1] * 45, [45], [20, 1, 1, 1, 22]):
+        s = _sim((4, 4), (16, 16))
+        s.set_option('chunks', 1)
+        s.add_species(-1.0, (3, 3), udist=('thermal', (0.1, 0.1, 0.1), (0, 0, 0.2)))
+        for n in parts:
+            s.advance(n)
+        runs.append((s.grid('E'), s.grid('B'), s.tiles(0)[0], s.iter()))
+    for r in runs[1:]:
+        for a, b in zip(runs[0], r):
+            assert np.array_equal(a, b)

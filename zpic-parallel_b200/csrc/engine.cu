@@ -52,6 +52,9 @@ cudaError_t launch_field_energy( cudaStream_t, const RunDev *, int, int, double 
 cudaError_t launch_grid_add( cudaStream_t, float *, const float *, size_t );
 cudaError_t launch_charge_finish( cudaStream_t, const float *, float *, int, int, int, int, int, int, int, int );
 cudaError_t launch_grid_gather( cudaStream_t, const float *, float *, int, int, int, int, int, int, int, int );
+void readback_retain( int );
+void readback_release( int );
+cudaError_t copy_to_host( int, cudaStream_t, void *, const void *, size_t );
 }  // namespace zb
 
 using namespace zb;
@@ -104,7 +107,11 @@ template < class T > static int dalloc( T ** p, size_t n ) {
 }
 template < class T > static void dfree( T *& p ) { if ( p ) cudaFree( p ); p = nullptr; }
 
+// doubles of a simulation's pinned scratch: values read back first, the status word last
+constexpr int HSCRATCH = 64, HS_STATUS = HSCRATCH - 1;
+
 static inline int roundup4( int n ) { return ( n + 3 ) & ~3; }
+constexpr int SINGLE_STEPS = 32;    // single-step calls before the step is captured in a graph
 constexpr int MAX_SPECIES = 64;     // species per simulation
 
 enum Phase { PH_PARTICLES = 0, PH_SORT, PH_CURRENT, PH_FIELDS, PH_OTHER, PH_N };
@@ -189,6 +196,7 @@ struct Plan {
     int reorder_every = 0;          // steps between in-tile reorders (option "reorder"; 0: never)
     int reorder_count = 0;          // steps since the last reorder
     bool needs_bc_or_filter = false;
+    int single_steps = 0;           // steps asked for one at a time so far (up to SINGLE_STEPS)
     cudaGraphExec_t graph = nullptr;
     int graph_kernels = 0;
     // in-graph phase timing (profile 2): the captured graph and its event-record
@@ -251,6 +259,8 @@ struct zpic_sim {
     double * fe_part_d = nullptr;  // per-tile field-energy partials (6 per tile), device
     double * fe_part_h = nullptr;  // and their pinned host copy, allocated on first use
     double * hscratch = nullptr;   // pinned host mirror
+    char * work_d = nullptr;       // kept device workspace of the diagnostics (Workspace)
+    size_t work_bytes = 0;
     int * shifts_d = nullptr;
     std::vector<HSpecies *> species;
     Plan plan;
@@ -294,11 +304,13 @@ static int sim_select( zpic_sim * s ) {
     return ZPIC_OK;
 }
 
-// Reads the kernels' status word.  A failure is reported once: the word is
-// cleared when it is read, so a later call starts clean (the state the
-// failed work left behind is not repaired).
+// Waits for the simulation's work and reads the kernels' status word (through
+// pinned memory, behind whatever copies the caller has queued: one wait for
+// all of them).  A failure is reported once: the word is cleared when it is
+// read, so a later call starts clean (the state the failed work left behind
+// is not repaired).
 static int check_status( zpic_sim * s ) {
-    int st = 0;
+    int & st = *reinterpret_cast<int *>( s->hscratch + HS_STATUS );
     CK( cudaMemcpyAsync( &st, s->status, sizeof( int ), cudaMemcpyDeviceToHost, s->stream ) );
     CK( cudaStreamSynchronize( s->stream ) );
     if ( st & ( ST_WAIT_TIMEOUT | ST_CAPACITY | ST_BAD_CELL ) ) {
@@ -312,6 +324,36 @@ static int check_status( zpic_sim * s ) {
     }
     return ZPIC_OK;
 }
+
+// Device workspace of one diagnostic call.  Up to the size of one vector grid
+// (1 MB at least) it is kept by the simulation from call to call; a larger one
+// is allocated for the call.  (An allocation and a free per call cost 0.2 ms
+// when the device was idle and up to 50 ms when its memory had just grown.)
+struct Workspace {
+    char * p = nullptr;
+    bool own = false;
+    size_t used = 0;
+    int get( zpic_sim * s, size_t bytes ) {
+        const size_t keep = std::max<size_t>( s->grid_floats() * sizeof( float ), 1 << 20 );
+        if ( bytes > keep ) { own = true; return dalloc( &p, bytes ); }
+        if ( bytes > s->work_bytes ) {
+            dfree( s->work_d );
+            s->work_bytes = 0;
+            TRY( dalloc( &s->work_d, bytes ) );
+            s->work_bytes = bytes;
+        }
+        p = s->work_d;
+        return ZPIC_OK;
+    }
+    // n elements from it, 256-byte aligned
+    template < class T > T * take( size_t n ) {
+        T * r = reinterpret_cast<T *>( p + used );
+        used += bytes_of<T>( n );
+        return r;
+    }
+    template < class T > static size_t bytes_of( size_t n ) { return ( std::max<size_t>( n, 1 ) * sizeof( T ) + 255 ) & ~(size_t) 255; }
+    ~Workspace() { if ( own ) dfree( p ); }
+};
 
 // Chunks (CTAs) per tile for the particle kernel: enough work items to fill
 // the GPU a few times over (the reference splits tiles over blockIdx.z the
@@ -680,7 +722,11 @@ static int maybe_reorder( Plan & P, cudaStream_t st, uint64_t * launches ) {
 
 static int plan_advance( Plan & P, cudaStream_t st, int nsteps, bool use_graph, uint64_t * launches ) {
     for ( auto * s : P.sims ) TRY( ensure_jdep_clean( s, st ) );
-    const bool can_graph = use_graph && nsteps > 1;
+    // a step is captured when several are asked for at once, or when single
+    // steps keep coming: capturing costs about 0.5 ms, a replay saves about
+    // 10 us of launches
+    if ( nsteps == 1 && P.single_steps < SINGLE_STEPS ) P.single_steps++;
+    const bool can_graph = use_graph && ( nsteps > 1 || P.graph || P.single_steps >= SINGLE_STEPS );
     zpic_sim * ts = prof_sim( P );
     const bool timing = ts && ts->profile == 2;
     if ( can_graph && P.graph && timing != !P.timed.empty() ) P.drop_step_graph();
@@ -1273,8 +1319,8 @@ int zpic_b200_sim_create( uint32_t ntx, uint32_t nty, uint32_t nxx, uint32_t nxy
     CK( cudaMemset( s->status, 0, sizeof( int ) ) );
     R.status = s->status;
     R.wait_limit = WAIT_LIMIT_DEFAULT;
-    TRY( dalloc( &s->dscratch, 64 ) );
-    CK( cudaMallocHost( (void **) &s->hscratch, 64 * sizeof( double ) ) );
+    TRY( dalloc( &s->dscratch, HSCRATCH ) );
+    CK( cudaMallocHost( (void **) &s->hscratch, HSCRATCH * sizeof( double ) ) );
     // cell shift of a moving-window step: -1 for whichever species the
     // particle kernel is launched for (at most MAX_SPECIES per simulation)
     TRY( dalloc( &s->shifts_d, MAX_SPECIES ) );
@@ -1283,6 +1329,7 @@ int zpic_b200_sim_create( uint32_t ntx, uint32_t nty, uint32_t nxx, uint32_t nxy
         CK( cudaMemcpy( s->shifts_d, neg.data(), MAX_SPECIES * sizeof( int ), cudaMemcpyHostToDevice ) );
     }
     TRY( upload_run( s.get() ) );
+    readback_retain( dev );
     *out = s.release();
     return ZPIC_OK;
 }
@@ -1298,7 +1345,9 @@ int zpic_b200_sim_destroy( zpic_sim * s ) {
     dfree( s->status ); dfree( s->dscratch ); dfree( s->shifts_d ); dfree( s->fe_part_d );
     if ( s->fe_part_h ) { cudaFreeHost( s->fe_part_h ); s->fe_part_h = nullptr; }
     if ( s->hscratch ) cudaFreeHost( s->hscratch );
+    dfree( s->work_d );
     cudaStreamDestroy( s->stream );
+    readback_release( s->device );
     delete s;
     return ZPIC_OK;
 }
@@ -1583,7 +1632,6 @@ int zpic_b200_sim_iter( zpic_sim * s, uint32_t * iter ) {
 
 int zpic_b200_sim_synchronize( zpic_sim * s ) {
     TRY( sim_select( s ) );
-    CK( cudaStreamSynchronize( s->stream ) );
     return check_status( s );
 }
 
@@ -1635,7 +1683,6 @@ int zpic_b200_emf_advance( zpic_sim * s, int32_t with_current ) {
         TRY( run_shift( s->plan, s->stream, 0 ) );
         s->emf_mw.advance();
     }
-    CK( cudaStreamSynchronize( s->stream ) );
     return check_status( s );
 }
 
@@ -1654,11 +1701,11 @@ int zpic_b200_emf_energy( zpic_sim * s, double ene_E[3], double ene_B[3] ) {
     s->launches++;
     const double * h = s->fe_part_h;
     CK( cudaMemcpyAsync( s->fe_part_h, s->fe_part_d, 6 * (size_t) nt * sizeof( double ), cudaMemcpyDeviceToHost, s->stream ) );
-    CK( cudaStreamSynchronize( s->stream ) );
+    const int rc = check_status( s );
     double e[6] = { 0, 0, 0, 0, 0, 0 };
     for ( int t = 0; t < nt; t++ ) for ( int k = 0; k < 6; k++ ) e[k] += h[6 * (size_t) t + k];   // tile order
     for ( int k = 0; k < 3; k++ ) { ene_E[k] = e[k]; ene_B[k] = e[3 + k]; }
-    return check_status( s );
+    return rc;
 }
 
 int zpic_b200_laser_add( zpic_sim * s, const zpic_laser_desc * l ) {
@@ -1714,7 +1761,6 @@ int zpic_b200_current_advance( zpic_sim * s ) {
     s->j_final = true;
     s->cur_iter++;
     if ( s->cur_mw.needs_move( s->cur_iter * s->dt ) ) s->cur_mw.advance();
-    CK( cudaStreamSynchronize( s->stream ) );
     return check_status( s );
 }
 
@@ -1788,11 +1834,10 @@ int zpic_b200_species_energy( zpic_sim * s, int32_t sp, double * energy ) {
     const int items = h->energy_items > 0 ? h->energy_items : h->ntiles * h->d.nchunk;
     CK( launch_energy_sum( s->stream, s->plan.sps_d, sp, items, s->dscratch ) );
     s->launches++;
-    double d = 0;
-    CK( cudaMemcpyAsync( &d, s->dscratch, sizeof( double ), cudaMemcpyDeviceToHost, s->stream ) );
-    CK( cudaStreamSynchronize( s->stream ) );
-    *energy = d * h->q * h->m_q * h->dx[0] * h->dx[1];          // species.h:365-368
-    return check_status( s );
+    CK( cudaMemcpyAsync( s->hscratch, s->dscratch, sizeof( double ), cudaMemcpyDeviceToHost, s->stream ) );
+    const int rc = check_status( s );
+    *energy = s->hscratch[0] * h->q * h->m_q * h->dx[0] * h->dx[1];          // species.h:365-368
+    return rc;
 }
 
 int zpic_b200_species_nmove( zpic_sim * s, int32_t sp, uint64_t * nmove ) {
@@ -1887,18 +1932,20 @@ int zpic_b200_species_get( zpic_sim * s, int32_t sp, int32_t * ix, float * x, fl
     std::vector<int> n, o;
     TRY( tiles_host( s, sp, n, o ) );
     const size_t total = (size_t) o.back() + n.back();
-    int * poff_d = nullptr; int2 * ix_d = nullptr; float2 * x_d = nullptr; float * u_d = nullptr;
-    TRY( dalloc( &poff_d, h->ntiles ) ); TRY( dalloc( &ix_d, total ) ); TRY( dalloc( &x_d, total ) ); TRY( dalloc( &u_d, 3 * total ) );
+    Workspace w;
+    TRY( w.get( s, w.bytes_of<int>( h->ntiles ) + w.bytes_of<int2>( total ) + w.bytes_of<float2>( total ) + w.bytes_of<float>( 3 * total ) ) );
+    int * poff_d = w.take<int>( h->ntiles );
+    int2 * ix_d = w.take<int2>( total );
+    float2 * x_d = w.take<float2>( total );
+    float * u_d = w.take<float>( 3 * total );
     CK( cudaMemcpyAsync( poff_d, o.data(), o.size() * sizeof( int ), cudaMemcpyHostToDevice, s->stream ) );
     CK( launch_pack( s->stream, sp, h->ntiles, s->plan.sps_d, poff_d, ix_d, x_d, u_d ) );
     s->launches++;
     if ( total ) {
-        CK( cudaMemcpyAsync( ix, ix_d, total * sizeof( int2 ), cudaMemcpyDeviceToHost, s->stream ) );
-        CK( cudaMemcpyAsync( x, x_d, total * sizeof( float2 ), cudaMemcpyDeviceToHost, s->stream ) );
-        CK( cudaMemcpyAsync( u, u_d, 3 * total * sizeof( float ), cudaMemcpyDeviceToHost, s->stream ) );
+        CK( copy_to_host( s->device, s->stream, ix, ix_d, total * sizeof( int2 ) ) );
+        CK( copy_to_host( s->device, s->stream, x, x_d, total * sizeof( float2 ) ) );
+        CK( copy_to_host( s->device, s->stream, u, u_d, 3 * total * sizeof( float ) ) );
     }
-    CK( cudaStreamSynchronize( s->stream ) );
-    dfree( poff_d ); dfree( ix_d ); dfree( x_d ); dfree( u_d );
     return check_status( s );
 }
 
@@ -1925,17 +1972,17 @@ int zpic_b200_species_gather( zpic_sim * s, int32_t sp, int32_t quant, float * o
     std::vector<int> n, o;
     TRY( tiles_host( s, sp, n, o ) );
     const size_t total = (size_t) o.back() + n.back();
-    int * poff_d = nullptr; float * out_d = nullptr;
-    TRY( dalloc( &poff_d, h->ntiles ) ); TRY( dalloc( &out_d, total ) );
+    Workspace w;
+    TRY( w.get( s, w.bytes_of<int>( h->ntiles ) + w.bytes_of<float>( total ) ) );
+    int * poff_d = w.take<int>( h->ntiles );
+    float * out_d = w.take<float>( total );
     CK( cudaMemcpyAsync( poff_d, o.data(), o.size() * sizeof( int ), cudaMemcpyHostToDevice, s->stream ) );
     // Species::gather scales positions by dx (species.h:510-526)
     const int scaled = quant <= 1;
     const float sx = quant == 0 ? h->dx[0] : h->dx[1];
     CK( launch_gather( s->stream, sp, h->ntiles, s->plan.sps_d, s->plan.runs_d, poff_d, quant, sx, 0.f, scaled, out_d ) );
     s->launches++;
-    if ( total ) CK( cudaMemcpyAsync( out, out_d, total * sizeof( float ), cudaMemcpyDeviceToHost, s->stream ) );
-    CK( cudaStreamSynchronize( s->stream ) );
-    dfree( poff_d ); dfree( out_d );
+    CK( copy_to_host( s->device, s->stream, out, out_d, total * sizeof( float ) ) );
     return ZPIC_OK;
 }
 
@@ -1947,16 +1994,16 @@ int zpic_b200_species_charge( zpic_sim * s, int32_t sp, float * out ) {
     const int cvol = roundup4( cextx * cexty );
     const size_t nraw = (size_t) cvol * h->ntiles;
     const size_t ndense = (size_t) s->ntx * s->nxx * s->nty * s->nxy;
-    float * raw = nullptr; float * dense = nullptr;
-    TRY( dalloc( &raw, nraw ) ); TRY( dalloc( &dense, ndense ) );
+    Workspace w;
+    TRY( w.get( s, w.bytes_of<float>( nraw ) + w.bytes_of<float>( ndense ) ) );
+    float * raw = w.take<float>( nraw );
+    float * dense = w.take<float>( ndense );
     CK( cudaMemsetAsync( raw, 0, nraw * sizeof( float ), s->stream ) );
     CK( launch_dep_charge( s->stream, sp, h->ntiles, s->plan.sps_d, s->plan.runs_d, raw, cextx, cvol ) );
     // the charge grid is a new grid object, hence periodic (grid.h:79)
     CK( launch_charge_finish( s->stream, raw, dense, s->ntx, s->nty, s->nxx, s->nxy, cextx, cvol, 1, 1 ) );
     s->launches += 2;
-    CK( cudaMemcpyAsync( out, dense, ndense * sizeof( float ), cudaMemcpyDeviceToHost, s->stream ) );
-    CK( cudaStreamSynchronize( s->stream ) );
-    dfree( raw ); dfree( dense );
+    CK( copy_to_host( s->device, s->stream, out, dense, ndense * sizeof( float ) ) );
     return ZPIC_OK;
 }
 
@@ -1999,14 +2046,13 @@ int zpic_b200_species_phasespace( zpic_sim * s, int32_t sp, int32_t quant0, cons
     p.r0 = r0[0]; p.rdx0 = size0 / ( r0[1] - r0[0] );
     if ( two ) { p.r1 = r1[0]; p.rdx1 = size1 / ( r1[1] - r1[0] ); }
     const size_t nbins = (size_t) size0 * ( two ? size1 : 1 );
-    float * d = nullptr;
-    TRY( dalloc( &d, nbins ) );
+    Workspace w;
+    TRY( w.get( s, w.bytes_of<float>( nbins ) ) );
+    float * d = w.take<float>( nbins );
     CK( cudaMemsetAsync( d, 0, nbins * sizeof( float ), s->stream ) );
     CK( launch_phasespace( s->stream, sp, h->ntiles, s->plan.sps_d, s->plan.runs_d, p, d ) );
     s->launches += 1;
-    CK( cudaMemcpyAsync( out, d, nbins * sizeof( float ), cudaMemcpyDeviceToHost, s->stream ) );
-    CK( cudaStreamSynchronize( s->stream ) );
-    dfree( d );
+    CK( copy_to_host( s->device, s->stream, out, d, nbins * sizeof( float ) ) );
     return check_status( s );
 }
 
@@ -2030,8 +2076,7 @@ int zpic_b200_grid_get( zpic_sim * s, int32_t which, float * out ) {
     TRY( sim_select( s ) );
     float * p = grid_ptr( s, which, true );
     if ( !p || !out ) return fail( ZPIC_E_INVALID, "invalid grid" );
-    CK( cudaMemcpyAsync( out, p, s->grid_floats() * sizeof( float ), cudaMemcpyDeviceToHost, s->stream ) );
-    CK( cudaStreamSynchronize( s->stream ) );
+    CK( copy_to_host( s->device, s->stream, out, p, s->grid_floats() * sizeof( float ) ) );
     return ZPIC_OK;
 }
 
@@ -2051,13 +2096,12 @@ int zpic_b200_grid_gather( zpic_sim * s, int32_t which, int32_t fc, float * out 
     float * p = grid_ptr( s, which, true );
     if ( !p || !out || fc < 0 || fc > 2 ) return fail( ZPIC_E_INVALID, "invalid grid" );
     const size_t n = (size_t) s->ntx * s->nxx * s->nty * s->nxy;
-    float * d = nullptr;
-    TRY( dalloc( &d, n ) );
+    Workspace w;
+    TRY( w.get( s, w.bytes_of<float>( n ) ) );
+    float * d = w.take<float>( n );
     CK( launch_grid_gather( s->stream, p, d, fc, s->ntx, s->nty, s->nxx, s->nxy, s->run.extx, s->run.gc_off, s->run.tile_vol ) );
     s->launches++;
-    CK( cudaMemcpyAsync( out, d, n * sizeof( float ), cudaMemcpyDeviceToHost, s->stream ) );
-    CK( cudaStreamSynchronize( s->stream ) );
-    dfree( d );
+    CK( copy_to_host( s->device, s->stream, out, d, n * sizeof( float ) ) );
     return ZPIC_OK;
 }
 

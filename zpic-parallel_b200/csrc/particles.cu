@@ -1471,21 +1471,27 @@ __global__ void k_phasespace( int sp, const SpDev * __restrict__ sps, const RunD
     }
 }
 
-// Per-item energy sums reduced per species in item order (deterministic).
-__global__ void k_energy_sum( const SpDev * __restrict__ sps, int sp, int nitems, double * __restrict__ out )
+// Per-item energy sums reduced per species in a fixed order: every thread's
+// items, then warp trees (a serial sum of the threads' 256 values took twice
+// as long as the rest of the kernel).
+__global__ void __launch_bounds__( 256 )
+k_energy_sum( const SpDev * __restrict__ sps, int sp, int nitems, double * __restrict__ out )
 {
-    const SpDev & S = sps[sp];
-    __shared__ double s[256];
+    const double * __restrict__ e = sps[sp].energy;
+    __shared__ double s[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double a = 0.0;
-    const int per = ( nitems + blockDim.x - 1 ) / blockDim.x;
-    const int i0 = threadIdx.x * per, i1 = min( nitems, i0 + per );
-    for ( int i = i0; i < i1; i++ ) a += S.energy[i];
-    s[ threadIdx.x ] = a;
+#pragma unroll 4
+    for ( int i = threadIdx.x; i < nitems; i += 256 ) a += e[i];
+#pragma unroll
+    for ( int o = 16; o > 0; o >>= 1 ) a += __shfl_down_sync( 0xffffffffu, a, o );
+    if ( lane == 0 ) s[ warp ] = a;
     __syncthreads();
-    if ( threadIdx.x == 0 ) {
-        double tot = 0.0;
-        for ( int i = 0; i < (int) blockDim.x; i++ ) tot += s[i];
-        *out = tot;
+    if ( warp == 0 ) {
+        a = lane < 8 ? s[ lane ] : 0.0;
+#pragma unroll
+        for ( int o = 4; o > 0; o >>= 1 ) a += __shfl_down_sync( 0xffffffffu, a, o );
+        if ( lane == 0 ) *out = a;
     }
 }
 
