@@ -41,9 +41,9 @@ cudaError_t launch_energy_sum( cudaStream_t, const SpDev *, int, int, double * )
 cudaError_t launch_np_stats( cudaStream_t, const SpDev *, int, unsigned long long * );
 cudaError_t launch_reorder( cudaStream_t, const Item *, int, const SpDev *, const RunDev *, int );
 cudaError_t launch_current_gc( cudaStream_t, const TileItem *, int, const RunDev *, int );
-cudaError_t launch_emf_gc( cudaStream_t, const TileItem *, int, const RunDev *, int, int, int );
+cudaError_t launch_emf_gc( cudaStream_t, const TileItem *, int, const RunDev *, int, int, int, int, int );
 cudaError_t launch_cur_gc( cudaStream_t, const TileItem *, int, const RunDev *, int, int );
-cudaError_t launch_yee( cudaStream_t, const TileItem *, int, const RunDev *, int, int, int, int, int );
+cudaError_t launch_yee( cudaStream_t, const TileItem *, int, const RunDev *, int, int, int, int );
 cudaError_t launch_emf_bc( cudaStream_t, const RunDev *, int, int, int );
 cudaError_t launch_cur_bc( cudaStream_t, const RunDev *, int, int, int );
 cudaError_t launch_kernel3( cudaStream_t, const TileItem *, int, const RunDev *, int, int, float, float, float, int );
@@ -196,6 +196,7 @@ struct Plan {
     int reorder_every = 0;          // steps between in-tile reorders (option "reorder"; 0: never)
     int reorder_count = 0;          // steps since the last reorder
     bool needs_bc_or_filter = false;
+    bool sum_in_yee = true;         // the field solve sums the deposits (run_current_fields)
     int single_steps = 0;           // steps asked for one at a time so far (up to SINGLE_STEPS)
     cudaGraphExec_t graph = nullptr;
     int graph_kernels = 0;
@@ -412,6 +413,7 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
     P.jacc = -1;
     P.tile_n = -1;
     P.needs_bc_or_filter = false;
+    P.sum_in_yee = true;
     int total_tiles = 0;
     for ( auto * s : sims ) for ( auto * sp : s->species ) { (void) sp; total_tiles += s->ntx * s->nty; }
     // a batch chooses its CTAs per tile from all of its tiles; a single
@@ -438,6 +440,8 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
         for ( int k = 0; k < 4; k++ )
             if ( s->emf_bc[k] > ZPIC_EMF_BC_PERIODIC || s->cur_bc[k] > ZPIC_CURRENT_BC_PERIODIC ) P.needs_bc_or_filter = true;
         if ( s->ftype != ZPIC_FILTER_NONE || s->emf_mw.active ) P.needs_bc_or_filter = true;
+        if ( s->ftype != ZPIC_FILTER_NONE || s->nxx < 3 || s->nxy < 3 ) P.sum_in_yee = false;
+        for ( int k = 0; k < 4; k++ ) if ( s->cur_bc[k] > ZPIC_CURRENT_BC_PERIODIC ) P.sum_in_yee = false;
     }
     for ( size_t r = 0; r < sims.size(); r++ ) {
         zpic_sim * s = sims[r];
@@ -616,21 +620,18 @@ static int run_current( Plan & P, cudaStream_t st ) {
 }
 
 // EMF::advance device part (emf.cpp:513-580 and 135-194): Yee, guard cells, bc.
+// jsrc: the current's source (launch_yee); clear: clear the raw deposits for
+// the next step.
 // with_shift: EMF::move_window (emf.cpp:120-129) follows at once in a run
 // without physical boundaries; the Yee kernel writes its tiles shifted and
 // the guard refresh completes the shift (two kernels instead of four).
-static int run_fields( Plan & P, cudaStream_t st, int with_j, int j_raw, int clear_jdep, bool with_shift = false ) {
-    if ( with_shift ) {
-        PhaseScope ps( prof_sim( P ), st, PH_FIELDS, 2 );
-        DEV( launch_yee( st, P.tile_items_d, P.n_tiles, P.runs_d, with_j, j_raw, clear_jdep, P.max_tile_vol, 1 ) );
-        DEV( launch_emf_gc( st, P.tile_items_d, P.n_tiles, P.runs_d, 3, P.max_guard, P.max_nxy ) );
-        return ZPIC_OK;
-    }
+static int run_fields( Plan & P, cudaStream_t st, int jsrc, int clear, bool with_shift = false ) {
     {
         PhaseScope ps( prof_sim( P ), st, PH_FIELDS, 2 );
-        DEV( launch_yee( st, P.tile_items_d, P.n_tiles, P.runs_d, with_j, j_raw, clear_jdep, P.max_tile_vol, 0 ) );
-        DEV( launch_emf_gc( st, P.tile_items_d, P.n_tiles, P.runs_d, 3, P.max_guard, 0 ) );
+        DEV( launch_yee( st, P.tile_items_d, P.n_tiles, P.runs_d, jsrc, P.max_tile_vol, with_shift, P.tile_n ) );
+        DEV( launch_emf_gc( st, P.tile_items_d, P.n_tiles, P.runs_d, 3, P.max_guard, with_shift ? P.max_nxy : 0, clear, P.tile_n ) );
     }
+    if ( with_shift ) return ZPIC_OK;
     if ( !P.needs_bc_or_filter ) return ZPIC_OK;
     for ( size_t r = 0; r < P.sims.size(); r++ ) {
         zpic_sim * s = P.sims[r];
@@ -653,8 +654,18 @@ static int run_shift( Plan & P, cudaStream_t st, int r ) {
     const int nt = P.sims[r]->ntx * P.sims[r]->nty;
     PhaseScope ps( prof_sim( P ), st, PH_FIELDS, 2 );
     DEV( launch_shift_left( st, P.tile_items_d + first, nt, P.runs_d, P.max_tile_vol ) );
-    DEV( launch_emf_gc( st, P.tile_items_d + first, nt, P.runs_d, 1, P.max_guard, 0 ) );
+    DEV( launch_emf_gc( st, P.tile_items_d + first, nt, P.runs_d, 1, P.max_guard, 0, 0, P.tile_n ) );
     return ZPIC_OK;
+}
+
+// Current::advance and EMF::advance of a step: the field solve sums the
+// deposits of the tiles itself where nothing comes in between (reflecting
+// boundaries of the current, filters) and the tiles are large enough for its
+// sum (3x3 cells).
+static int run_current_fields( Plan & P, cudaStream_t st, bool with_shift ) {
+    if ( P.sum_in_yee ) return run_fields( P, st, 3, 1, with_shift );
+    TRY( run_current( P, st ) );
+    return run_fields( P, st, 1, 1, with_shift );
 }
 
 static int ensure_plan( zpic_sim * s ) {
@@ -677,8 +688,7 @@ static int plan_step_device( Plan & P, cudaStream_t st ) {
     // stream (forked after the particle kernel, joined before the step ends)
     DEV( cudaEventRecord( P.fork, st ) );
     DEV( cudaStreamWaitEvent( P.side, P.fork, 0 ) );
-    TRY( run_current( P, P.side ) );
-    TRY( run_fields( P, P.side, 1, 0, 1 ) );
+    TRY( run_current_fields( P, P.side, false ) );
     DEV( cudaEventRecord( P.join, P.side ) );
     TRY( run_sort( P, st, 0 ) );
     DEV( cudaStreamWaitEvent( st, P.join, 0 ) );
@@ -1535,7 +1545,6 @@ static int mw_step( zpic_sim * s ) {
     Plan & P = s->plan;
     DEV( cudaEventRecord( P.fork, s->stream ) );
     DEV( cudaStreamWaitEvent( P.side, P.fork, 0 ) );
-    TRY( run_current( P, P.side ) );
     s->cur_iter++;
     if ( s->cur_mw.needs_move( s->cur_iter * s->dt ) ) s->cur_mw.advance();
     // a window shift right after the field solve is folded into it (the Yee
@@ -1547,7 +1556,7 @@ static int mw_step( zpic_sim * s ) {
     const bool shift = s->emf_mw.active && s->emf_mw.needs_move( ( s->emf_iter + 1 ) * s->dt );
     bool fused = shift && P.sims.size() == 1 && s->run.emf_pery;
     for ( int k = 0; k < 4; k++ ) fused = fused && s->emf_bc[k] <= ZPIC_EMF_BC_PERIODIC;
-    TRY( run_fields( P, P.side, 1, 0, 1, fused ) );
+    TRY( run_current_fields( P, P.side, fused ) );
     s->jdep_clean = true;
     s->j_final = true;
     s->emf_iter++;
@@ -1677,7 +1686,7 @@ int zpic_b200_emf_set_bc( zpic_sim * s, const int32_t bc[4] ) {
 int zpic_b200_emf_advance( zpic_sim * s, int32_t with_current ) {
     TRY( sim_select( s ) );
     TRY( ensure_plan( s ) );
-    TRY( run_fields( s->plan, s->stream, with_current ? 1 : 0, s->j_final ? 0 : 1, 0 ) );
+    TRY( run_fields( s->plan, s->stream, !with_current ? 0 : s->j_final ? 1 : 2, 0 ) );
     s->emf_iter++;
     if ( s->emf_mw.active && s->emf_mw.needs_move( s->emf_iter * s->dt ) ) {
         TRY( run_shift( s->plan, s->stream, 0 ) );

@@ -130,10 +130,46 @@ k_current_gc( const TileItem * __restrict__ items, const RunDev * __restrict__ r
     }
 }
 
+// Tile shape: compile time for TN x TN tiles (every index division is then a
+// multiplication), else from the run descriptor.
+template < int TN > struct Shape {
+    int nxx, nxy, extx, exty, tv, gc;
+    __device__ __forceinline__ Shape( const RunDev & R )
+        : nxx( TN ? TN : R.nxx ), nxy( TN ? TN : R.nxy ), extx( TN ? TN + 3 : R.extx ), exty( TN ? TN + 3 : R.exty ),
+          tv( TN ? ( ( TN + 3 ) * ( TN + 3 ) + 3 ) & ~3 : R.tile_vol ), gc( TN ? TN + 4 : R.gc_off ) {}
+};
+
 // the tile right of (tx, ty) for E and B, or -1
 __device__ __forceinline__ int right_tile( const RunDev & R, int tx, int ty ) {
     const int n = nbr( tx + 1, R.ntx, R.emf_perx );
     return n >= 0 ? ty * R.ntx + n : -1;
+}
+
+// Guard cell g of a tile and its source, as resolve_copy gives it.
+template < int TN >
+__device__ __forceinline__ bool guard_source( int g, const RunDev & R, const Shape<TN> & sh, int perx, int pery, int axes,
+                                              int tx, int ty, int & i, int & j, int & stx, int & sty, int & si, int & sj ) {
+    const int bottom = GL * sh.extx, top = GU * sh.extx;
+    if ( g < bottom + top ) {
+        j = g / sh.extx; i = g - j * sh.extx;
+        if ( j >= GL ) j += sh.nxy;
+    } else {
+        const int q = g - bottom - top, r = q / ( GL + GU ), c = q - r * ( GL + GU );
+        j = GL + r;
+        i = c < GL ? c : sh.nxx + c;
+    }
+    stx = tx; sty = ty; si = i; sj = j;
+    if ( axes & 2 ) {
+        const int d = j < GL ? -1 : j >= GL + sh.nxy ? 1 : 0;
+        const int n = d ? nbr( ty + d, R.nty, pery ) : -1;
+        if ( n >= 0 ) { sty = n; sj = j - d * sh.nxy; }
+    }
+    if ( axes & 1 ) {
+        const int d = i < GL ? -1 : i >= GL + sh.nxx ? 1 : 0;
+        const int n = d ? nbr( tx + d, R.ntx, perx ) : -1;
+        if ( n >= 0 ) { stx = n; si = i - d * sh.nxx; }
+    }
+    return stx != tx || sty != ty;
 }
 
 // grid::copy_to_gc on E and B in place (axes: 1 x, 2 y, 3 both).
@@ -142,39 +178,55 @@ __device__ __forceinline__ int right_tile( const RunDev & R, int tx, int ty ) {
 // neighbour's first interior column saved in bcol (where there is a right
 // neighbour): the threads after the guard cells of a tile write it, and guard
 // cells whose source is such a cell read it from bcol as well.
+// clear: the tile's threads also clear its raw deposits for the next step
+// (every tile's current has been summed by the kernel before).
+//
+// Bound by the latency of its small scattered copies and, in the general
+// form, by the divisions of its index arithmetic: 16x16 tiles have their own
+// instance.  Field half of a step on 8,192 of them (vacuum, 2048x1024 cells),
+// sum, solve and guard copies: 105 us as three kernels with the general
+// arithmetic, 82 us as two.
+template < int TN >
 __global__ void __launch_bounds__( GC_THREADS )
-k_emf_gc( const TileItem * __restrict__ items, int nitems, int per, const RunDev * __restrict__ runs, int axes,
-          int bfix )
+k_emf_gc( const TileItem * __restrict__ items, int nitems, int per_, const RunDev * __restrict__ runs, int axes,
+          int bfix, int clear )
 {
+    constexpr int NG = TN ? ( TN + 3 ) * ( TN + 3 ) - TN * TN : 1;
     const unsigned gid = blockIdx.x * blockDim.x + threadIdx.x;     // n * per < 2^31 (launcher)
-    const int w = (int) ( gid / (unsigned) per ), g = (int) ( gid % (unsigned) per );
+    const unsigned per = TN ? ( bfix ? NG + TN : NG ) : per_;
+    const int w = (int) ( TN && !bfix ? gid / NG : gid / per );
+    const int g = (int) ( gid - w * per );
     if ( w >= nitems ) return;
     const TileItem it = items[w];
     const RunDev & R = runs[ it.run ];
+    const Shape<TN> sh( R );
     const int tx = it.tile % R.ntx, ty = it.tile / R.ntx;
-    const int ng = guard_count( R );
+    const int ng = TN ? NG : guard_count( R );
+    if ( clear && g < ng ) {
+        float4 * z = reinterpret_cast<float4 *>( R.Jdep + (size_t) it.tile * 3 * sh.tv );
+        for ( int q = g; q < 3 * sh.tv / 4; q += ng ) z[q] = make_float4( 0.f, 0.f, 0.f, 0.f );
+    }
     if ( g >= ng ) {
         const int row = g - ng;
-        if ( !bfix || row >= R.nxy ) return;
+        if ( !bfix || row >= sh.nxy ) return;
         const int rn = right_tile( R, tx, ty );
         if ( rn < 0 ) return;
-        const size_t dst = ( (size_t) it.tile * R.tile_vol + ( GL + row ) * R.extx + GL + R.nxx - 1 ) * 3;
-        const float * b = R.bcol + ( (size_t) rn * R.nxy + row ) * 3;
+        const size_t dst = ( (size_t) it.tile * sh.tv + ( GL + row ) * sh.extx + GL + sh.nxx - 1 ) * 3;
+        const float * b = R.bcol + ( (size_t) rn * sh.nxy + row ) * 3;
         const float b0 = b[0], b1 = b[1], b2 = b[2];
         R.B[dst] = b0; R.B[dst + 1] = b1; R.B[dst + 2] = b2;
         return;
     }
-    int i, j;
-    guard_cell( g, R, i, j );
-    int stx, sty, si, sj;
-    resolve_copy( R, R.emf_perx, R.emf_pery, axes, tx, ty, i, j, stx, sty, si, sj );
-    if ( stx == tx && sty == ty && si == i && sj == j ) return;
-    const size_t dst = ( (size_t) it.tile * R.tile_vol + j * R.extx + i ) * 3;
-    const float * e = cellp( R.E, R, stx, sty, si, sj );
-    const float * b = cellp( R.B, R, stx, sty, si, sj );
-    if ( bfix && si == GL + R.nxx - 1 && sj >= GL && sj < GL + R.nxy ) {
+    int i, j, stx, sty, si, sj;
+    if ( !guard_source<TN>( g, R, sh, R.emf_perx, R.emf_pery, axes, tx, ty, i, j, stx, sty, si, sj ) &&
+         si == i && sj == j ) return;
+    const size_t dst = ( (size_t) it.tile * sh.tv + j * sh.extx + i ) * 3;
+    const size_t src = ( (size_t) ( sty * R.ntx + stx ) * sh.tv + sj * sh.extx + si ) * 3;
+    const float * e = R.E + src;
+    const float * b = R.B + src;
+    if ( bfix && si == GL + sh.nxx - 1 && sj >= GL && sj < GL + sh.nxy ) {
         const int rn = right_tile( R, stx, sty );
-        if ( rn >= 0 ) b = R.bcol + ( (size_t) rn * R.nxy + sj - GL ) * 3;
+        if ( rn >= 0 ) b = R.bcol + ( (size_t) rn * sh.nxy + sj - GL ) * 3;
     }
     const float e0 = e[0], e1 = e[1], e2 = e[2], b0 = b[0], b1 = b[1], b2 = b[2];
     R.E[dst] = e0; R.E[dst + 1] = e1; R.E[dst + 2] = e2;
@@ -207,14 +259,14 @@ k_cur_gc( const TileItem * __restrict__ items, int nitems, int per, const RunDev
 // Yee solver (emf.cpp:513-580): per tile, E, B and J tiles staged into shared
 // memory with bulk asynchronous copies; B half step over [-1,nx], E step with
 // J over [0,nx+1], B half step; E and B tiles stored back with bulk copies.
-// The raw deposit buffer of the tile is cleared for the next step.
 // ---------------------------------------------------------------------------
-constexpr int YEE_THREADS = 256;
+constexpr int YEE_THREADS = 192;              // two passes over the 18x18 cells of a 16x16 tile, ten CTAs per SM
 
-__device__ __forceinline__ void yee_b_smem( const float * E, float * B, const RunDev & R, float dtx, float dty ) {
-    const int ys = R.extx;
-    const int w = R.nxx + 2, h = R.nxy + 2;
-    for ( int c = threadIdx.x; c < w * h; c += blockDim.x ) {
+template < int TN >
+__device__ __forceinline__ void yee_b_smem( const float * E, float * B, const Shape<TN> & sh, float dtx, float dty ) {
+    const int ys = sh.extx;
+    const int w = sh.nxx + 2, h = sh.nxy + 2;
+    for ( int c = threadIdx.x; c < w * h; c += YEE_THREADS ) {
         const int ix = c % w - 1, iy = c / w - 1;
         const int k = 3 * ( ix + iy * ys ), kx = 3 * ( ix + 1 + iy * ys ), ky = 3 * ( ix + ( iy + 1 ) * ys );
         B[k + 0] += ( -dty * ( E[ky + 2] - E[k + 2] ) );
@@ -223,11 +275,12 @@ __device__ __forceinline__ void yee_b_smem( const float * E, float * B, const Ru
     }
 }
 
-__device__ __forceinline__ void yee_e_smem( float * E, const float * B, const float * J, const RunDev & R,
+template < int TN >
+__device__ __forceinline__ void yee_e_smem( float * E, const float * B, const float * J, const Shape<TN> & sh,
                                             float dtx, float dty, float dt, int with_j ) {
-    const int ys = R.extx;
-    const int w = R.nxx + 2, h = R.nxy + 2;
-    for ( int c = threadIdx.x; c < w * h; c += blockDim.x ) {
+    const int ys = sh.extx;
+    const int w = sh.nxx + 2, h = sh.nxy + 2;
+    for ( int c = threadIdx.x; c < w * h; c += YEE_THREADS ) {
         const int ix = c % w, iy = c / w;
         const int k = 3 * ( ix + iy * ys ), kx = 3 * ( ix - 1 + iy * ys ), ky = 3 * ( ix + ( iy - 1 ) * ys );
         if ( with_j ) {
@@ -242,41 +295,106 @@ __device__ __forceinline__ void yee_e_smem( float * E, const float * B, const fl
     }
 }
 
+// J: where the current comes from.  J_NONE, J_FINAL (R.J), J_RAW (R.Jdep as it
+// is), or J_SUM: the raw deposits of this tile and its neighbours are summed
+// here, into shared memory for the solver and into R.J (guard cells included)
+// for whoever reads the current -- one kernel and one read of J less than a
+// separate sum (Current::advance, current.cpp:227-233).  For tiles of at least
+// 3x3 cells: then every cell of the block takes at most one neighbour's value
+// per axis, (own + x neighbour) + (y neighbour + diagonal), and these
+// two-term sums are the same floats whichever tile evaluates them.  The
+// neighbours' values are loaded before the wait for the tile's own copies.
+enum { J_NONE = 0, J_FINAL = 1, J_RAW = 2, J_SUM = 3 };
+
+template < int TN, int JSRC >
 __global__ void __launch_bounds__( YEE_THREADS )
-k_yee( const TileItem * __restrict__ items, const RunDev * __restrict__ runs, int with_j, int j_raw, int clear_jdep,
-       int shift_out )
+k_yee( const TileItem * __restrict__ items, const RunDev * __restrict__ runs, int shift_out )
 {
     extern __shared__ __align__( 16 ) unsigned char smem_raw[];
     const TileItem it = items[ blockIdx.x ];
     const RunDev & R = runs[ it.run ];
-    const int tv = R.tile_vol;
+    const Shape<TN> sh( R );
+    const int tv = sh.tv;
     float * sE = reinterpret_cast<float *>( smem_raw );
     float * sB = sE + 3 * tv;
     float * sJ = sB + 3 * tv;
     uint64_t * bar = reinterpret_cast<uint64_t *>( sJ + 3 * tv );
     const size_t toff = (size_t) it.tile * 3 * tv;
     const uint32_t bytes = 12u * tv;
-    const float * Jsrc = j_raw ? R.Jdep : R.J;
 
-    if ( threadIdx.x == 0 ) { mbar_init( bar, 1 ); fence_mbar_init(); }
-    __syncthreads();
     if ( threadIdx.x == 0 ) {
-        mbar_arrive_expect_tx( bar, with_j ? 3 * bytes : 2 * bytes );
+        mbar_init( bar, 1 );
+        fence_mbar_init();
+        mbar_arrive_expect_tx( bar, JSRC != J_NONE ? 3 * bytes : 2 * bytes );
         bulk_g2s( sE, R.E + toff, bytes, bar );
         bulk_g2s( sB, R.B + toff, bytes, bar );
-        if ( with_j ) bulk_g2s( sJ, Jsrc + toff, bytes, bar );
+        if ( JSRC != J_NONE ) bulk_g2s( sJ, ( JSRC == J_FINAL ? R.J : R.Jdep ) + toff, bytes, bar );
     }
+    constexpr int NB = TN ? ( ( TN + 3 ) * ( TN + 3 ) + YEE_THREADS - 1 ) / YEE_THREADS : 1;
+    float xn[NB][3], yd[NB][3];
+    // one cell's neighbour sums (zeros where there is no neighbour)
+    auto neighbours = [&]( int c, float x[3], float y[3] ) {
+        x[0] = x[1] = x[2] = y[0] = y[1] = y[2] = 0.f;
+        const int j = c / sh.extx, i = c - j * sh.extx;
+        const int dx = i < GL + GU ? -1 : i >= sh.nxx ? 1 : 0, dy = j < GL + GU ? -1 : j >= sh.nxy ? 1 : 0;
+        if ( dx == 0 && dy == 0 ) return;
+        const int tx = it.tile % R.ntx, ty = it.tile / R.ntx;
+        const int ntx = dx ? nbr( tx + dx, R.ntx, R.cur_perx ) : -1, nty = dy ? nbr( ty + dy, R.nty, R.cur_pery ) : -1;
+        const int cx = c - dx * sh.nxx, cy = c - dy * sh.nxy * sh.extx, cd = cy - dx * sh.nxx;
+        if ( ntx >= 0 ) {
+            const float * q = R.Jdep + ( (size_t) ( ty * R.ntx + ntx ) * tv + cx ) * 3;
+            x[0] = q[0]; x[1] = q[1]; x[2] = q[2];
+        }
+        if ( nty >= 0 ) {
+            const float * q = R.Jdep + ( (size_t) ( nty * R.ntx + tx ) * tv + cy ) * 3;
+            y[0] = q[0]; y[1] = q[1]; y[2] = q[2];
+            if ( ntx >= 0 ) {
+                const float * d = R.Jdep + ( (size_t) ( nty * R.ntx + ntx ) * tv + cd ) * 3;
+                y[0] += d[0]; y[1] += d[1]; y[2] += d[2];
+            }
+        }
+    };
+    const int ncell = sh.extx * sh.exty;
+    if constexpr ( JSRC == J_SUM && TN > 0 ) {
+#pragma unroll
+        for ( int n = 0; n < NB; n++ ) {
+            const int c = threadIdx.x + n * YEE_THREADS;
+            if ( c < ncell ) neighbours( c, xn[n], yd[n] );
+        }
+    }
+    __syncthreads();
     // an expired wait: no field update and no stores for this tile
     if ( bulk_wait_or_abandon( bar, R.status, R.wait_limit ) ) return;
 
-    float * E0 = sE + 3 * R.gc_off;
-    float * B0 = sB + 3 * R.gc_off;
-    const float * J0 = sJ + 3 * R.gc_off;
-    yee_b_smem( E0, B0, R, R.dtx2, R.dty2 );
+    float * E0 = sE + 3 * sh.gc;
+    float * B0 = sB + 3 * sh.gc;
+    const float * J0 = sJ + 3 * sh.gc;
+    yee_b_smem<TN>( E0, B0, sh, R.dtx2, R.dty2 );
+    if constexpr ( JSRC == J_SUM ) {
+        auto sum = [&]( int c, const float x[3], const float y[3] ) {
+#pragma unroll
+            for ( int k = 0; k < 3; k++ ) sJ[ 3 * c + k ] = ( sJ[ 3 * c + k ] + x[k] ) + y[k];
+        };
+        if constexpr ( TN > 0 ) {
+#pragma unroll
+            for ( int n = 0; n < NB; n++ ) {
+                const int c = threadIdx.x + n * YEE_THREADS;
+                if ( c < ncell ) sum( c, xn[n], yd[n] );
+            }
+        } else {
+            for ( int c = threadIdx.x; c < ncell; c += YEE_THREADS ) { neighbours( c, xn[0], yd[0] ); sum( c, xn[0], yd[0] ); }
+        }
+    }
     __syncthreads();
-    yee_e_smem( E0, B0, J0, R, R.dtx, R.dty, R.dt, with_j );
+    if ( JSRC == J_SUM && threadIdx.x == 0 ) {
+        fence_proxy_async_smem();
+        bulk_s2g( R.J + toff, sJ, bytes );
+        bulk_commit();
+    }
+    yee_e_smem<TN>( E0, B0, J0, sh, R.dtx, R.dty, R.dt, JSRC != J_NONE );
     __syncthreads();
-    yee_b_smem( E0, B0, R, R.dtx2, R.dty2 );
+    yee_b_smem<TN>( E0, B0, sh, R.dtx2, R.dty2 );
+    if ( shift_out && JSRC == J_SUM && threadIdx.x == 0 ) bulk_wait_read_all();      // the shifted E takes J's place
     __syncthreads();
 
     const float * outE = sE, * outB = sB;
@@ -290,30 +408,26 @@ k_yee( const TileItem * __restrict__ items, const RunDev * __restrict__ runs, in
         // need E one column further out, so the first interior column of B is
         // saved (bcol) and the guard refresh that follows (k_emf_gc, bfix)
         // puts the right neighbour's in place, refreshing every guard cell.
-        float * dst = R.bcol + (size_t) it.tile * R.nxy * 3;
-        for ( int q = threadIdx.x; q < 3 * R.nxy; q += blockDim.x ) dst[q] = B0[ 3 * ( ( q / 3 ) * R.extx ) + q % 3 ];
-        const int ys = R.extx, nc = 3 * R.extx * R.exty;
+        float * dst = R.bcol + (size_t) it.tile * sh.nxy * 3;
+        for ( int q = threadIdx.x; q < 3 * sh.nxy; q += YEE_THREADS ) dst[q] = B0[ 3 * ( ( q / 3 ) * sh.extx ) + q % 3 ];
+        const int row = 3 * sh.extx, nc = row * sh.exty;
         float * sT = sJ;
-        for ( int e = threadIdx.x; e < 3 * tv; e += blockDim.x )
-            sT[e] = e < nc ? ( ( ( e / 3 ) % ys < ys - 1 ) ? sE[ e + 3 ] : 0.0f ) : sE[e];
+        for ( int e = threadIdx.x; e < 3 * tv; e += YEE_THREADS )
+            sT[e] = e < nc ? ( e % row < row - 3 ? sE[ e + 3 ] : 0.0f ) : sE[e];
         __syncthreads();
-        for ( int e = threadIdx.x; e < 3 * tv; e += blockDim.x )
-            sE[e] = e < nc ? ( ( ( e / 3 ) % ys < ys - 1 ) ? sB[ e + 3 ] : 0.0f ) : sB[e];
+        for ( int e = threadIdx.x; e < 3 * tv; e += YEE_THREADS )
+            sE[e] = e < nc ? ( e % row < row - 3 ? sB[ e + 3 ] : 0.0f ) : sB[e];
         __syncthreads();
         outE = sT; outB = sE;
     }
+    // the shared-memory sources read; the stores complete before the kernel does
     if ( threadIdx.x == 0 ) {
         fence_proxy_async_smem();
         bulk_s2g( R.E + toff, outE, bytes );
         bulk_s2g( R.B + toff, outB, bytes );
         bulk_commit();
+        bulk_wait_read_all();
     }
-    if ( clear_jdep ) {
-        float4 * z = reinterpret_cast<float4 *>( R.Jdep + toff );
-        for ( int i = threadIdx.x; i < 3 * tv / 4; i += blockDim.x ) z[i] = make_float4( 0.f, 0.f, 0.f, 0.f );
-    }
-    // the shared-memory sources read; the stores complete before the kernel does
-    if ( threadIdx.x == 0 ) bulk_wait_read_all();
 }
 
 // ---------------------------------------------------------------------------
@@ -646,11 +760,14 @@ cudaError_t launch_current_gc( cudaStream_t st, const TileItem * items, int n, c
     if ( n > 0 ) k_current_gc<<< n, 128, 0, st >>>( items, runs );
     return cudaGetLastError();
 }
+// tile_n: 16 when every tile is 16x16
 cudaError_t launch_emf_gc( cudaStream_t st, const TileItem * items, int n, const RunDev * runs, int axes, int per,
-                           int bfix_rows ) {
+                           int bfix_rows, int clear, int tile_n ) {
     per += bfix_rows;
     if ( !gc_fits( n, per ) ) return cudaErrorInvalidConfiguration;
-    if ( n > 0 ) k_emf_gc<<< gc_blocks( n, per ), GC_THREADS, 0, st >>>( items, n, per, runs, axes, bfix_rows > 0 );
+    if ( n > 0 )
+        ( tile_n == 16 ? k_emf_gc<16> : k_emf_gc<0> )<<< gc_blocks( n, per ), GC_THREADS, 0, st >>>( items, n, per, runs, axes,
+                                                                                                  bfix_rows > 0, clear );
     return cudaGetLastError();
 }
 cudaError_t launch_cur_gc( cudaStream_t st, const TileItem * items, int n, const RunDev * runs, int axes, int per ) {
@@ -658,11 +775,16 @@ cudaError_t launch_cur_gc( cudaStream_t st, const TileItem * items, int n, const
     if ( n > 0 ) k_cur_gc<<< gc_blocks( n, per ), GC_THREADS, 0, st >>>( items, n, per, runs, axes );
     return cudaGetLastError();
 }
-cudaError_t launch_yee( cudaStream_t st, const TileItem * items, int n, const RunDev * runs,
-                        int with_j, int j_raw, int clear_jdep, int max_tile_vol, int shift_out ) {
+// jsrc: 0 no current, 1 R.J, 2 raw deposits, 3 raw deposits summed over the tiles into R.J
+cudaError_t launch_yee( cudaStream_t st, const TileItem * items, int n, const RunDev * runs, int jsrc, int max_tile_vol,
+                        int shift_out, int tile_n ) {
+    typedef void ( *fn )( const TileItem *, const RunDev *, int );
+    static const fn f16[4] = { k_yee< 16, 0 >, k_yee< 16, 1 >, k_yee< 16, 2 >, k_yee< 16, 3 > };
+    static const fn f0[4] = { k_yee< 0, 0 >, k_yee< 0, 1 >, k_yee< 0, 2 >, k_yee< 0, 3 > };
+    const fn f = ( tile_n == 16 ? f16 : f0 )[ jsrc ];
     const size_t smem = yee_smem_bytes( max_tile_vol );
-    if ( smem > 48 * 1024 ) cudaFuncSetAttribute( (const void *) k_yee, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem );
-    if ( n > 0 ) k_yee<<< n, YEE_THREADS, smem, st >>>( items, runs, with_j, j_raw, clear_jdep, shift_out );
+    if ( smem > 48 * 1024 ) cudaFuncSetAttribute( (const void *) f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem );
+    if ( n > 0 ) f<<< n, YEE_THREADS, smem, st >>>( items, runs, shift_out );
     return cudaGetLastError();
 }
 cudaError_t launch_emf_bc( cudaStream_t st, const RunDev * runs, int run, int axis, int nthreads ) {
