@@ -28,7 +28,7 @@ size_t particle_smem_bytes( int tile_vol, int jacc );
 size_t yee_smem_bytes( int tile_vol );
 cudaError_t launch_particles( cudaStream_t, int, int, int, const Item *, int, const SpDev *, const RunDev *, const int *,
                               int, int, int );
-cudaError_t launch_sort( cudaStream_t, const Item *, int, const SpDev *, const int *, int, const RunDev *, int, int * );
+cudaError_t launch_sort( cudaStream_t, const Item *, int, const SegItem *, int, const SpDev *, const RunDev *, int, int *, int, long long, int );
 cudaError_t launch_inject( cudaStream_t, int, int, int, int, int, const SpDev *, const RunDev *, const InjRule &, int );
 cudaError_t launch_inj_dyn( cudaStream_t, float *, unsigned *, int, float, float, float, double );
 cudaError_t launch_pack( cudaStream_t, int, int, const SpDev *, const int *, int2 *, float2 *, float * );
@@ -181,11 +181,13 @@ struct Plan {
     std::vector<int> sp_sim, sp_local;          // plan species -> (sim index, species index)
     Item * k1_items_d[2] = { nullptr, nullptr }; int n_k1[2] = { 0, 0 };   // boris, euler
     Item * sort_items_d = nullptr; int n_sort = 0;
-    int * splist_d = nullptr; int n_sp = 0;
-    int * rlist_d = nullptr;        // [1 + n_sp] species repacking in the current sort (count, then indices)
+    SegItem * segs_d = nullptr; int n_segs = 0;     // the sort check's work, species by species
+    int n_sp = 0;
+    long long max_part = 0;         // particle capacity of all species
+    int * rlist_d = nullptr;        // [2 + n_sp] species repacking in the current sort (count, indices, a CTA count)
     // the same work lists grouped per species (fine-grained species calls)
     Item * spk1_d = nullptr;
-    std::vector<int> sp_k1_off, sp_k1_n, sp_sort_off, sp_sort_n;
+    std::vector<int> sp_k1_off, sp_k1_n, sp_sort_off, sp_sort_n, sp_seg_off, sp_seg_n;
     TileItem * tile_items_d = nullptr; int n_tiles = 0;
     int max_tile_vol = 0;
     int max_cells = 0, max_guard = 0;   // cells and guard cells of the largest tile
@@ -229,7 +231,7 @@ struct Plan {
         for ( auto & g : mw_graphs ) cudaGraphExecDestroy( g.second.first );
         mw_graphs.clear();
         dfree( runs_d ); dfree( sps_d ); dfree( k1_items_d[0] ); dfree( k1_items_d[1] );
-        dfree( sort_items_d ); dfree( splist_d ); dfree( rlist_d ); dfree( tile_items_d ); dfree( spk1_d );
+        dfree( sort_items_d ); dfree( segs_d ); dfree( rlist_d ); dfree( tile_items_d ); dfree( spk1_d );
         built = false;
     }
 };
@@ -403,10 +405,10 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
     P.sims = sims;
     std::vector<RunDev> runs;
     std::vector<Item> k1[2], sort_items, spk1;
-    std::vector<int> splist;
+    std::vector<SegItem> segs;
     std::vector<TileItem> tiles;
     P.sps_h.clear(); P.sp_sim.clear(); P.sp_local.clear();
-    P.sp_k1_off.clear(); P.sp_k1_n.clear(); P.sp_sort_off.clear(); P.sp_sort_n.clear();
+    P.sp_k1_off.clear(); P.sp_k1_n.clear(); P.sp_sort_off.clear(); P.sp_sort_n.clear(); P.sp_seg_off.clear(); P.sp_seg_n.clear();
     P.max_tile_vol = 0;
     P.max_cells = 0; P.max_guard = 0; P.max_tile_cells = 0; P.max_nxy = 0;
     P.reorder_every = 0; P.reorder_count = 0;
@@ -453,7 +455,9 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
             const int gi = (int) P.sps_h.size();
             P.sps_h.push_back( d );
             P.sp_sim.push_back( (int) r ); P.sp_local.push_back( (int) k );
-            splist.push_back( gi );
+            P.sp_seg_off.push_back( (int) segs.size() );
+            for ( int t = 0; t < sp->ntiles; t += SEG_TILES ) segs.push_back( { gi, t } );
+            P.sp_seg_n.push_back( (int) segs.size() - P.sp_seg_off.back() );
             P.sp_k1_off.push_back( (int) spk1.size() );
             P.sp_sort_off.push_back( (int) sort_items.size() );
             for ( int t = 0; t < sp->ntiles; t++ ) {
@@ -467,12 +471,14 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
             P.sp_sort_n.push_back( (int) sort_items.size() - P.sp_sort_off.back() );
         }
     }
-    P.n_sp = (int) splist.size();
+    P.n_sp = (int) P.sps_h.size();
+    P.max_part = 0;
+    for ( auto & d : P.sps_h ) P.max_part += d.max_part;
     TRY( dalloc( &P.runs_d, runs.size() ) );
     TRY( dalloc( &P.sps_d, P.sps_h.size() ) );
-    TRY( dalloc( &P.splist_d, splist.size() ) );
-    TRY( dalloc( &P.rlist_d, splist.size() + 1 ) );
-    CK( cudaMemset( P.rlist_d, 0, ( splist.size() + 1 ) * sizeof( int ) ) );
+    TRY( dalloc( &P.segs_d, segs.size() ) );
+    TRY( dalloc( &P.rlist_d, P.n_sp + 2 ) );
+    CK( cudaMemset( P.rlist_d, 0, ( P.n_sp + 2 ) * sizeof( int ) ) );
     TRY( dalloc( &P.tile_items_d, tiles.size() ) );
     TRY( dalloc( &P.sort_items_d, sort_items.size() ) );
     CK( cudaStreamCreateWithFlags( &P.side, cudaStreamNonBlocking ) );
@@ -481,7 +487,7 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
     CK( cudaMemcpy( P.runs_d, runs.data(), runs.size() * sizeof( RunDev ), cudaMemcpyHostToDevice ) );
     if ( !P.sps_h.empty() ) {
         CK( cudaMemcpy( P.sps_d, P.sps_h.data(), P.sps_h.size() * sizeof( SpDev ), cudaMemcpyHostToDevice ) );
-        CK( cudaMemcpy( P.splist_d, splist.data(), splist.size() * sizeof( int ), cudaMemcpyHostToDevice ) );
+        CK( cudaMemcpy( P.segs_d, segs.data(), segs.size() * sizeof( SegItem ), cudaMemcpyHostToDevice ) );
         CK( cudaMemcpy( P.sort_items_d, sort_items.data(), sort_items.size() * sizeof( Item ), cudaMemcpyHostToDevice ) );
     }
     CK( cudaMemcpy( P.tile_items_d, tiles.data(), tiles.size() * sizeof( TileItem ), cudaMemcpyHostToDevice ) );
@@ -495,6 +501,7 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
     if ( !spk1.empty() )
         CK( cudaMemcpy( P.spk1_d, spk1.data(), spk1.size() * sizeof( Item ), cudaMemcpyHostToDevice ) );
     P.n_sort = (int) sort_items.size();
+    P.n_segs = (int) segs.size();
     P.n_tiles = (int) tiles.size();
     P.built = true;
     return ZPIC_OK;
@@ -569,8 +576,12 @@ static int run_particles( Plan & P, cudaStream_t st, int push, int move, const i
 
 static int run_sort( Plan & P, cudaStream_t st, int use_extra ) {
     if ( P.n_sp == 0 ) return ZPIC_OK;
-    PhaseScope ps( prof_sim( P ), st, PH_SORT, 4 );
-    DEV( launch_sort( st, P.sort_items_d, P.n_sort, P.sps_d, P.splist_d, P.n_sp, P.runs_d, use_extra, P.rlist_d ) );
+    PhaseScope ps( prof_sim( P ), st, PH_SORT, 3 );
+    // behind the particle kernel, unless timing events lie in between
+    const zpic_sim * timed = prof_sim( P );
+    const int overlap = !( timed && timed->profile );
+    DEV( launch_sort( st, P.sort_items_d, P.n_sort, P.segs_d, P.n_segs, P.sps_d, P.runs_d, use_extra, P.rlist_d, P.n_sp,
+                      P.max_part, overlap ) );
     return ZPIC_OK;
 }
 
@@ -966,14 +977,14 @@ static int species_alloc( zpic_sim * s, HSpecies * sp, uint64_t max_part ) {
     TRY( dalloc( &d.idx, max_part ) ); TRY( dalloc( &d.aux, max_part ) ); TRY( dalloc( &d.aux2, max_part ) );
     TRY( dalloc( &d.in_cnt, nt ) ); TRY( dalloc( &d.stage_cnt, nt ) );
     TRY( dalloc( &d.cnt, 9 * (size_t) nt ) ); TRY( dalloc( &d.base, 9 * (size_t) nt ) );
-    TRY( dalloc( &d.hs, nt ) ); TRY( dalloc( &d.overflow, 1 ) );
+    TRY( dalloc( &d.hs, nt ) ); TRY( dalloc( &d.overflow, 2 ) );
     TRY( dalloc( &d.reloc, nt ) ); TRY( dalloc( &d.pool, 1 ) );
     TRY( dalloc( &d.rel_tile, nt ) ); TRY( dalloc( &d.rel_start, nt + 1 ) ); TRY( dalloc( &d.rel_n, 1 ) );
     CK( cudaMemset( d.rel_n, 0, sizeof( int ) ) );
     CK( cudaMemset( d.reloc, 0, nt * sizeof( int ) ) );
     CK( cudaMemset( d.pool, 0, sizeof( int ) ) );
     CK( cudaMemset( d.cnt, 0, 9 * (size_t) nt * sizeof( int ) ) );
-    CK( cudaMemset( d.overflow, 0, sizeof( int ) ) );
+    CK( cudaMemset( d.overflow, 0, 2 * sizeof( int ) ) );
     TRY( dalloc( &d.new_off, nt ) ); TRY( dalloc( &d.new_cap, nt ) ); TRY( dalloc( &d.new_np, nt ) );
     TRY( dalloc( &d.extra, nt ) ); TRY( dalloc( &d.mode, 1 ) );
     TRY( dalloc( &sp->inj_dyn, 4 ) ); TRY( dalloc( &sp->mw_nmove_d, 1 ) );
@@ -1148,9 +1159,9 @@ static int species_sort( zpic_sim * s, int sp, int use_extra ) {
                               nullptr, P.max_tile_vol, 0, 0 ) );
     }
     {
-        PhaseScope ps( s, s->stream, PH_SORT, 4 );
-        DEV( launch_sort( s->stream, P.sort_items_d + P.sp_sort_off[sp], P.sp_sort_n[sp], P.sps_d,
-                         P.splist_d + sp, 1, P.runs_d, use_extra, P.rlist_d ) );
+        PhaseScope ps( s, s->stream, PH_SORT, 3 );
+        DEV( launch_sort( s->stream, P.sort_items_d + P.sp_sort_off[sp], P.sp_sort_n[sp], P.segs_d + P.sp_seg_off[sp],
+                          P.sp_seg_n[sp], P.sps_d, P.runs_d, use_extra, P.rlist_d, P.n_sp, h->max_part, 0 ) );
     }
     h->sort_pending = false;
     h->counters_dirty = false;

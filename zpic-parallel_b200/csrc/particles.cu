@@ -354,6 +354,7 @@ k_particles( const Item * __restrict__ items, const SpDev * __restrict__ sps,
              const RunDev * __restrict__ runs, const int * __restrict__ shifts )
 {
     extern __shared__ __align__( 16 ) unsigned char smem_raw[];
+    dep_launch();                               // the sort's check may be set up behind the last wave of this kernel
     const Item it = items[ blockIdx.x ];
     const SpDev & S = sps[ it.sp ];
     const RunDev & R = runs[ S.run ];
@@ -668,9 +669,10 @@ k_particles( const Item * __restrict__ items, const SpDev * __restrict__ sps,
 // d = 3 (ycross + 1) + xcross + 1, 4 meaning "stays").  Then:
 //   k_sort_check   per tile: incoming per direction from the 8 neighbour
 //                  counts, their offsets (base), the new count, and whether
-//                  it fits the tile's slot;
-//   k_sort_plan    per species: in place (mode 0) if every tile fits, else
-//                  a new slot layout (mode 1, a repack through buffer B);
+//                  it fits the tile's slot; the last of a species' CTAs then
+//                  plans the species: in place (mode 0) if every tile fits,
+//                  else new slots for those that do not (mode 3) or a new slot
+//                  layout (mode 1, a repack through buffer B);
 //   k_sort_local   per tile: the slots that are empty below the new count
 //                  (leavers' slots, or room after the old count) are listed;
 //                  stayers above the new count move into the first of them,
@@ -689,72 +691,84 @@ __device__ __forceinline__ int neighbor_tile( int t, int d, int ntx, int nty, in
     return ( wx >= 0 && wy >= 0 ) ? wy * ntx + wx : -1;
 }
 
-constexpr int CHECK_THREADS = 256;
-
-// One thread per (species, tile) item.  Particles arriving at t through
-// direction d come from the neighbour in the opposite direction 8 - d.
-__global__ void __launch_bounds__( CHECK_THREADS )
-k_sort_check( const Item * __restrict__ items, int nitems, const SpDev * __restrict__ sps,
-              const RunDev * __restrict__ runs, int use_extra, int * __restrict__ rlist )
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if ( i == 0 ) rlist[0] = 0;                   // the plan lists the species that repack
-    if ( i >= nitems ) return;
-    const Item it = items[i];
-    const SpDev & S = sps[ it.sp ];
-    const RunDev & R = runs[ S.run ];
-    const int t = it.tile;
-    int g[9];
-#pragma unroll
-    for ( int d = 0; d < 9; d++ ) {
-        const int src = d == 4 ? -1 : neighbor_tile( t, 8 - d, R.ntx, R.nty, S.perx, S.pery );
-        g[d] = src >= 0 ? S.cnt[ 9 * src + d ] : 0;
-    }
-    int in = 0;
-#pragma unroll
-    for ( int d = 0; d < 9; d++ ) { S.base[ 9 * t + d ] = in; in += g[d]; }
-    const int stay = S.np[t] - S.nidx[t];
-    const int ex = ( use_extra && S.extra ) ? S.extra[t] : 0;
-    S.in_cnt[t] = in;
-    S.new_np[t] = stay + in;
-    int rel = 0;
-    if ( stay + in + ex > S.cap[t] ) {
-        // a new slot in the pool, with room to grow (reloc_room times its
-        // count, at least twice the minimum slack): a tile that outgrew its
-        // slot is usually still growing
-        rel = 1;
-        atomicAdd( S.nmove + 2, 1ull );
-        const int grow = max( 2 * S.min_slack, (int) ( S.reloc_room * ( stay + in ) ) );
-        S.new_cap[t] = ( ( stay + in + ex + 3 ) & ~3 ) + ( ( grow + 3 ) & ~3 );
-        atomicOr( S.overflow, 1 );
-    }
-    S.reloc[t] = rel;
-}
-
-constexpr int PLAN_THREADS = 1024;
+constexpr int PLAN_THREADS = SEG_TILES;
 // rlist entries: species index, with this bit set for a species that only
 // relocates tiles (mode 3) rather than repacking (mode 1)
 constexpr int RLIST_RELOCATE = 1 << 30;
 
-// One CTA per species.  In place (mode 0) unless a tile overflowed its slot;
-// then the repack layout (mode 1): need[t] = new count + injection reserve,
-// rounded up to 4, and the free capacity spread in proportion to
-// need + min_slack (multiples of 4); mode 2 when the buffer cannot hold the
-// new total (ST_CAPACITY: the host grows buffers before that can happen).
-__global__ void __launch_bounds__( PLAN_THREADS )
-k_sort_plan( const SpDev * __restrict__ sps, const int * __restrict__ species_list,
-             const RunDev * __restrict__ runs, int use_extra, int * __restrict__ rlist )
-{
-    const SpDev & S = sps[ species_list[ blockIdx.x ] ];
-    const RunDev & R = runs[ S.run ];
-    const int over = *S.overflow;
-    __syncthreads();
+__device__ __noinline__ void sort_plan( int sp, const SpDev & S, const RunDev & R, int use_extra, int * __restrict__ rlist );
 
-    if ( !over ) {
-        if ( threadIdx.x == 0 ) *S.mode = 0;
-        return;
+// One thread per tile, one CTA per SEG_TILES tiles of a species.  Particles
+// arriving at t through direction d come from the neighbour in the opposite
+// direction 8 - d.  The CTA that finishes a species' last segment plans it (a
+// kernel of its own for that cost 4-5 us of every step, nearly always to find
+// that no tile overflowed).
+__global__ void __launch_bounds__( SEG_TILES )
+k_sort_check( const SegItem * __restrict__ segs, const SpDev * __restrict__ sps,
+              const RunDev * __restrict__ runs, int use_extra, int * __restrict__ rlist )
+{
+    const SegItem sg = segs[ blockIdx.x ];
+    const SpDev & S = sps[ sg.sp ];
+    const RunDev & R = runs[ S.run ];
+    const int t = sg.tile + threadIdx.x, ntx = R.ntx, nty = R.nty;
+    dep_wait();
+    dep_launch();
+    bool over = false;
+    if ( t < S.ntiles ) {
+        int g[9];
+        const int tx = t % ntx, ty = t / ntx;
+#pragma unroll
+        for ( int d = 0; d < 9; d++ ) {
+            const int wx = wrap_tile( tx + 1 - d % 3, ntx, S.perx ), wy = wrap_tile( ty + 1 - d / 3, nty, S.pery );
+            g[d] = d != 4 && wx >= 0 && wy >= 0 ? S.cnt[ 9 * ( wy * ntx + wx ) + d ] : 0;
+        }
+        int in = 0;
+#pragma unroll
+        for ( int d = 0; d < 9; d++ ) { S.base[ 9 * t + d ] = in; in += g[d]; }
+        const int stay = S.np[t] - S.nidx[t];
+        const int ex = ( use_extra && S.extra ) ? S.extra[t] : 0;
+        S.in_cnt[t] = in;
+        S.new_np[t] = stay + in;
+        over = stay + in + ex > S.cap[t];
+        if ( over ) {
+            // a new slot in the pool, with room to grow (reloc_room times its
+            // count, at least twice the minimum slack): a tile that outgrew its
+            // slot is usually still growing
+            atomicAdd( S.nmove + 2, 1ull );
+            const int grow = max( 2 * S.min_slack, (int) ( S.reloc_room * ( stay + in ) ) );
+            S.new_cap[t] = ( ( stay + in + ex + 3 ) & ~3 ) + ( ( grow + 3 ) & ~3 );
+        }
+        S.reloc[t] = over;
     }
-    if ( threadIdx.x == 0 ) *S.overflow = 0;
+    const int any = __syncthreads_or( over );
+    __shared__ int s_plan;                        // -1: not the last segment; else whether any tile overflowed
+    if ( threadIdx.x == 0 ) {
+        if ( any ) atomicOr( S.overflow, 1 );
+        __threadfence();
+        const int nseg = ( S.ntiles + SEG_TILES - 1 ) / SEG_TILES;
+        s_plan = -1;
+        if ( atomicAdd( S.overflow + 1, 1 ) == nseg - 1 ) {
+            __threadfence();
+            s_plan = atomicExch( S.overflow, 0 );
+            S.overflow[1] = 0;
+            if ( !s_plan ) *S.mode = 0;
+        }
+    }
+    __syncthreads();
+    if ( s_plan > 0 ) {
+        __threadfence();
+        sort_plan( sg.sp, S, R, use_extra, rlist );
+    }
+}
+
+// By one CTA, for a species with tiles that overflowed their slots: new slots
+// from the pool for those (mode 3), or the repack layout (mode 1): need[t] =
+// new count + injection reserve, rounded up to 4, and the free capacity spread
+// in proportion to need + min_slack (multiples of 4); mode 2 when the buffer
+// cannot hold the new total (ST_CAPACITY: the host grows buffers before that
+// can happen).
+__device__ __noinline__ void sort_plan( int sp, const SpDev & S, const RunDev & R, int use_extra, int * __restrict__ rlist )
+{
     const int nt = S.ntiles;
     const int per = ( nt + PLAN_THREADS - 1 ) / PLAN_THREADS;
     const int t0 = min( nt, (int) threadIdx.x * per ), t1 = min( nt, t0 + per );
@@ -788,7 +802,7 @@ k_sort_plan( const SpDev * __restrict__ sps, const int * __restrict__ species_li
             if ( threadIdx.x == 0 ) {
                 *S.pool = (int) ( pool + rtotal ); *S.mode = 3;
                 S.rel_start[ nrel ] = (int) ptotal; *S.rel_n = (int) nrel;
-                rlist[ 1 + atomicAdd( rlist, 1 ) ] = species_list[ blockIdx.x ] | RLIST_RELOCATE;
+                rlist[ 1 + atomicAdd( rlist, 1 ) ] = sp | RLIST_RELOCATE;
             }
             return;
         }
@@ -835,7 +849,7 @@ k_sort_plan( const SpDev * __restrict__ sps, const int * __restrict__ species_li
         *S.pool = (int) s_total;
         *S.mode = 1;
         S.nmove[1] += 1;
-        rlist[ 1 + atomicAdd( rlist, 1 ) ] = species_list[ blockIdx.x ];
+        rlist[ 1 + atomicAdd( rlist, 1 ) ] = sp;
     }
 }
 
@@ -981,6 +995,10 @@ k_sort_local( const Item * __restrict__ items, int nitems, const SpDev * __restr
     if ( active ) {
         it = items[ wi ];
         Sp = &sps[ it.sp ];
+    }
+    dep_wait();
+    dep_launch();
+    if ( active ) {
         if ( sub == 0 && lane < 9 ) Sp->cnt[ 9 * it.tile + lane ] = 0;
         const int mode = *Sp->mode;
         active = mode == 0 || mode == 3;
@@ -1087,7 +1105,7 @@ k_sort_local( const Item * __restrict__ items, int nitems, const SpDev * __restr
 template < int WPT >
 __global__ void __launch_bounds__( SORT_THREADS )
 k_sort_scatter( const Item * __restrict__ items, int nitems, const SpDev * __restrict__ sps,
-                const int * __restrict__ rlist, const RunDev * __restrict__ runs )
+                int * __restrict__ rlist, int nsp, const RunDev * __restrict__ runs )
 {
     constexpr int TPB = SORT_WARPS / WPT;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1107,6 +1125,9 @@ k_sort_scatter( const Item * __restrict__ items, int nitems, const SpDev * __res
     if ( active ) {
         it = items[ wi ];
         Sp = &sps[ it.sp ];
+    }
+    dep_wait();
+    if ( active ) {
         mode = *Sp->mode;
         active = mode == 0 || mode == 3;
     }
@@ -1201,6 +1222,13 @@ k_sort_scatter( const Item * __restrict__ items, int nitems, const SpDev * __res
     const int nr = rlist[0];
     for ( int k = 0; k < nr; k++ )
         if ( !( rlist[ 1 + k ] & RLIST_RELOCATE ) ) repack_in( sps[ rlist[ 1 + k ] ] );
+    // the last CTA empties the list for the next sort (its CTA count follows
+    // the nsp entries)
+    __syncthreads();
+    if ( threadIdx.x == 0 ) {
+        __threadfence();
+        if ( atomicAdd( rlist + 1 + nsp, 1 ) == (int) gridDim.x - 1 ) { rlist[ 1 + nsp ] = 0; rlist[0] = 0; }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1724,29 +1752,46 @@ cudaError_t launch_particles( cudaStream_t st, int push, int move, int detect, c
     return cudaGetLastError();
 }
 
-cudaError_t launch_sort( cudaStream_t st, const Item * items, int nitems, const SpDev * sps,
-                         const int * species_list, int nspecies, const RunDev * runs, int use_extra, int * rlist ) {
+// The kernels of a sort are launched so that each is set up (and has read its
+// work item) while the one before it drains.  overlap_first: so is the check
+// behind the particle kernel; only when that is the stream's previous work.
+// max_part: capacity of the species sorted.
+template < class... P, class... A >
+static cudaError_t launch_after( cudaStream_t st, bool overlap, void ( *f )( P... ), int grid, int threads, A... args ) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3( grid ); c.blockDim = dim3( threads ); c.stream = st;
+    cudaLaunchAttribute a{};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &a;
+    c.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx( &c, f, static_cast<P>( args )... );
+}
+
+// rlist: [count][nsp entries][CTAs of the scatter kernel done]
+cudaError_t launch_sort( cudaStream_t st, const Item * items, int nitems, const SegItem * segs, int nsegs, const SpDev * sps,
+                         const RunDev * runs, int use_extra, int * rlist, int nsp, long long max_part, int overlap_first ) {
     if ( nitems <= 0 ) return cudaSuccess;
     int dev = 0, sms = 148;
     cudaGetDevice( &dev );
     cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
-    k_sort_check<<< ( nitems + CHECK_THREADS - 1 ) / CHECK_THREADS, CHECK_THREADS, 0, st >>>( items, nitems, sps, runs,
-                                                                                         use_extra, rlist );
-    k_sort_plan<<< nspecies, PLAN_THREADS, 0, st >>>( sps, species_list, runs, use_extra, rlist );
+    cudaError_t e = launch_after( st, overlap_first != 0, k_sort_check, nsegs, SEG_TILES, segs, sps, runs, use_extra, rlist );
     // a warp per tile, unless the tiles are too few to occupy the GPU's SMs
-    // (then they are large, and get a CTA each); the grid covers the GPU at
-    // least once for the repack's grid-stride loops
+    // (then they are large, and get a CTA each); more CTAs than that only for
+    // the grid-stride loops of a repack, by the particles there may be to move:
+    // idle CTAs of the two kernels, resident at the same time, would keep the
+    // field half off the SMs (592 of each: 65 instead of 59 us per step of a
+    // filtered 256x64 wakefield)
     const bool wide = nitems < sms * 16;
     const int tpb = wide ? 1 : SORT_WARPS;
-    const int nb = std::max( ( nitems + tpb - 1 ) / tpb, 4 * sms );
-    if ( wide ) {
-        k_sort_local< SORT_WARPS ><<< nb, SORT_THREADS, 0, st >>>( items, nitems, sps, rlist, runs );
-        k_sort_scatter< SORT_WARPS ><<< nb, SORT_THREADS, 0, st >>>( items, nitems, sps, rlist, runs );
-    } else {
-        k_sort_local< 1 ><<< nb, SORT_THREADS, 0, st >>>( items, nitems, sps, rlist, runs );
-        k_sort_scatter< 1 ><<< nb, SORT_THREADS, 0, st >>>( items, nitems, sps, rlist, runs );
-    }
-    return cudaGetLastError();
+    const int nb = std::max( ( nitems + tpb - 1 ) / tpb, std::min( 4 * sms, (int) ( max_part / 4096 ) ) );
+    if ( e == cudaSuccess )
+        e = launch_after( st, true, wide ? k_sort_local< SORT_WARPS > : k_sort_local< 1 >, nb, SORT_THREADS, items, nitems, sps,
+                          rlist, runs );
+    if ( e == cudaSuccess )
+        e = launch_after( st, true, wide ? k_sort_scatter< SORT_WARPS > : k_sort_scatter< 1 >, nb, SORT_THREADS, items, nitems,
+                          sps, rlist, nsp, runs );
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_inj_dyn( cudaStream_t st, float * dyn, unsigned * n_move, int type, float da, float db,

@@ -69,7 +69,7 @@ struct SpDev {
     int * in_cnt;                 // [ntiles] incoming particles (sort check)
     int * hs;                     // [ntiles] stayers moved down inside the tile (sort); in a repack:
                                   // packed position of each tile's first particle, old layout
-    int * overflow;               // [1] a tile's new count exceeds its slot (sort check)
+    int * overflow;               // [2] a tile's new count exceeds its slot (sort check); segments checked so far
     int * reloc;                  // [ntiles] 1: the tile outgrew its slot and moves to the pool (sort check)
     int * pool;                   // [1] start of the free pool after the last slot (pool ends at max_part)
     int * rel_tile;               // [ntiles] relocated tiles of the current sort, in tile order (plan)
@@ -213,6 +213,16 @@ __device__ __forceinline__ int cell_y( uint32_t c ) { return static_cast<int>( s
 
 // Work item of the particle kernels: species, tile, chunk
 struct Item { int sp; int tile; int chunk; int pad; };
+
+// Tiles [tile, tile + SEG_TILES) of a species: work item of the sort's check.
+constexpr int SEG_TILES = 1024;
+struct SegItem { int sp; int tile; };
+
+// Programmatic launches: wait for the kernel this one depends on (complete,
+// its writes visible); let the kernel that depends on this one be set up.
+// Both do nothing in a kernel launched without the attribute.
+__device__ __forceinline__ void dep_wait() { asm volatile( "griddepcontrol.wait;" ::: "memory" ); }
+__device__ __forceinline__ void dep_launch() { asm volatile( "griddepcontrol.launch_dependents;" ::: "memory" ); }
 
 // Phase-space deposit parameters (quantities 0 x, 1 y, 2 ux, 3 uy, 4 uz;
 // q1 < 0 for a 1D phase space).  r = lower range bound in deposit units,
