@@ -358,16 +358,35 @@ struct Workspace {
     ~Workspace() { if ( own ) dfree( p ); }
 };
 
-// Chunks (CTAs) per tile for the particle kernel: enough work items to fill
-// the GPU a few times over (the reference splits tiles over blockIdx.z the
-// same way, cuda/em2d/species.cpp:924-937).
-static int auto_chunks( int ntiles_total, int opt ) {
+// Chunks (CTAs) per tile for the particle kernel (the reference splits tiles
+// over blockIdx.z the same way, cuda/em2d/species.cpp:924-937), by the time a
+// launch would take: its waves of resident CTAs (per_sm of them on an SM),
+// each CTA with its fixed part (set-up, field staging, write-back of the tile
+// current) and its particles, plus the cost of every CTA launched.  Measured:
+// 10.3 ns per particle in a full wave, 5 us fixed, 8.2 ns per CTA.  Small runs
+// get one full wave rather than two and a bit (128x128 Weibel set-up, 4 CTAs
+// per tile instead of 10: 41 against 47 us per step while it is uniform; 64x64
+// cells 33 -> 26 us), few large tiles several (512 tiles of 32x32 cells, 6
+// instead of 3: 861 -> 831 us).
+static int auto_chunks( uint64_t ntiles, double particles_per_tile, int per_sm, int opt ) {
     if ( opt > 0 ) return opt;
     int dev = 0; cudaGetDevice( &dev );
     int sms = 148; cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
-    const int target = sms * 8;
-    if ( ntiles_total >= target ) return 1;
-    return std::min( 64, ( target + ntiles_total - 1 ) / ntiles_total );
+    const double slots = (double) sms * per_sm;
+    int best = 1; double best_us = 0;
+    for ( int c = 1; c <= 64; c++ ) {
+        const double ctas = (double) ntiles * c;
+        const double us = std::ceil( ctas / slots ) * ( 0.0103 * particles_per_tile / c + 5.0 ) + 0.0082 * ctas;
+        if ( c == 1 || us < best_us ) { best = c; best_us = us; }
+    }
+    return best;
+}
+
+// Particles per tile of a full plasma, and CTAs of the particle kernel per SM
+// (64 registers a thread allow four; large tiles fewer by their shared memory).
+static double nominal_per_tile( const zpic_sim * s, const HSpecies * h ) { return (double) h->ppc[0] * h->ppc[1] * s->nxx * s->nxy; }
+static int ctas_per_sm( const zpic_sim * s ) {
+    return std::max( 1, std::min( 4, (int) ( 227 * 1024 / ( particle_smem_bytes( s->run.tile_vol, s->jacc ) + 1024 ) ) ) );
 }
 
 // CTAs per tile of the particle kernel ("chunks" option): n > 0 for every
@@ -378,9 +397,9 @@ static int auto_chunks( int ntiles_total, int opt ) {
 // plasma fills the tiles (faster once a Weibel plasma has filamented, slower
 // for uniform plasmas and for runs with many empty tiles).
 static void set_chunks( zpic_sim * s ) {
-    int ntot = 0; uint64_t np = 0;
-    for ( auto * h : s->species ) { ntot += h->ntiles; np += h->np_bound; }
-    const int base = auto_chunks( std::max( 1, ntot ), std::max( 0, s->chunks_opt ) );
+    int ntot = 0; uint64_t np = 0; double nominal = 0;
+    for ( auto * h : s->species ) { ntot += h->ntiles; np += h->np_bound; nominal += h->ntiles * nominal_per_tile( s, h ); }
+    const int base = auto_chunks( std::max( 1, ntot ), nominal / std::max( 1, ntot ), ctas_per_sm( s ), std::max( 0, s->chunks_opt ) );
     for ( auto * h : s->species ) {
         if ( s->chunks_opt >= 0 ) { h->d.nchunk = base; h->d.chunk_target = 0; continue; }
         h->d.nchunk = std::min( 64, 2 * base );
@@ -416,12 +435,15 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
     P.tile_n = -1;
     P.needs_bc_or_filter = false;
     P.sum_in_yee = true;
-    int total_tiles = 0;
-    for ( auto * s : sims ) for ( auto * sp : s->species ) { (void) sp; total_tiles += s->ntx * s->nty; }
+    uint64_t total_tiles = 0; double nominal = 0; int per_sm = 4;
+    for ( auto * s : sims ) {
+        per_sm = std::min( per_sm, ctas_per_sm( s ) );
+        for ( auto * sp : s->species ) { total_tiles += sp->ntiles; nominal += sp->ntiles * nominal_per_tile( s, sp ); }
+    }
     // a batch chooses its CTAs per tile from all of its tiles; a single
     // simulation keeps the choice made for it
     const int batch_chunks = chunks_override > 0 ? chunks_override
-                           : sims.size() > 1 ? auto_chunks( std::max( 1, total_tiles ), 0 ) : 0;
+                           : sims.size() > 1 ? auto_chunks( std::max<uint64_t>( 1, total_tiles ), nominal / std::max<uint64_t>( 1, total_tiles ), per_sm, 0 ) : 0;
     for ( size_t r = 0; r < sims.size(); r++ ) {
         zpic_sim * s = sims[r];
         runs.push_back( s->run );
@@ -1242,12 +1264,11 @@ static int species_advance_mw( zpic_sim * s, int sp ) {
 // real steps of the simulation(s).  The physics does not depend on the
 // choice; only the order in which the per-CTA partial currents are added to
 // the raw current (FP32) does.
-static std::vector<int> chunk_candidates( uint64_t particles, uint64_t tiles, int automatic ) {
+static std::vector<int> chunk_candidates( uint64_t particles, uint64_t tiles ) {
     std::vector<int> c;
     const double per_tile = tiles ? (double) particles / tiles : 0.0;
     for ( int k = 1; k <= 64; k *= 2 )
         if ( k == 1 || per_tile / k >= 256.0 ) c.push_back( k );
-    (void) automatic;
     c.insert( c.begin(), -1 );
     c.insert( c.begin(), 0 );
     return c;
@@ -2187,9 +2208,8 @@ int zpic_b200_sim_autotune( zpic_sim * s, int32_t steps, int32_t * chosen ) {
     if ( s->species.empty() ) return fail( ZPIC_E_INVALID, "no species to tune for" );
     if ( s->emf_mw.active ) return fail( ZPIC_E_INVALID, "autotune runs Simulation::advance steps; not for moving-window runs" );
     uint64_t ntiles = 0; for ( auto * h : s->species ) ntiles += h->ntiles;
-    const int automatic = auto_chunks( (int) ntiles, 0 );
-    int best = automatic; float best_ms = -1;
-    for ( int c : chunk_candidates( particles_of( s ), ntiles, automatic ) ) {
+    int best = 0; float best_ms = -1;
+    for ( int c : chunk_candidates( particles_of( s ), ntiles ) ) {
         TRY( zpic_b200_sim_set_option( s, "chunks", c ) );
         float ms = 0;
         TRY( time_candidate( s->stream, steps, [&]( int n ) { return zpic_b200_sim_advance( s, n ); }, &ms ) );
@@ -2206,9 +2226,8 @@ int zpic_b200_batch_autotune( zpic_batch * b, int32_t steps, int32_t * chosen ) 
     CK( cudaSetDevice( b->sims[0]->device ) );
     uint64_t ntiles = 0, np = 0;
     for ( auto * s : b->sims ) { np += particles_of( s ); for ( auto * h : s->species ) ntiles += h->ntiles; }
-    const int automatic = auto_chunks( (int) std::min<uint64_t>( ntiles, 1u << 30 ), 0 );
-    int best = automatic; float best_ms = -1;
-    for ( int c : chunk_candidates( np, ntiles, automatic ) ) {
+    int best = 0; float best_ms = -1;
+    for ( int c : chunk_candidates( np, ntiles ) ) {
         if ( c < 0 ) continue;          // a batch chunks all of its runs alike
         b->chunks = c;
         TRY( plan_build( b->plan, b->sims, c ) );
