@@ -47,6 +47,8 @@ cudaError_t launch_yee( cudaStream_t, const TileItem *, int, const RunDev *, int
 cudaError_t launch_emf_bc( cudaStream_t, const RunDev *, int, int, int );
 cudaError_t launch_cur_bc( cudaStream_t, const RunDev *, int, int, int );
 cudaError_t launch_kernel3( cudaStream_t, const TileItem *, int, const RunDev *, int, int, float, float, float, int );
+size_t filter_smem_bytes( int, int, int, int );
+cudaError_t launch_filter( cudaStream_t, const TileItem *, int, const RunDev *, int, int, const float *, const float *, size_t );
 cudaError_t launch_shift_left( cudaStream_t, const TileItem *, int, const RunDev *, int );
 cudaError_t launch_field_energy( cudaStream_t, const RunDev *, int, int, double * );
 cudaError_t launch_grid_add( cudaStream_t, float *, const float *, size_t );
@@ -199,6 +201,7 @@ struct Plan {
     int reorder_count = 0;          // steps since the last reorder
     bool needs_bc_or_filter = false;
     bool sum_in_yee = true;         // the field solve sums the deposits (run_current_fields)
+    bool filter_in_one = true;      // every run has a current filter that one kernel takes (run_current)
     int single_steps = 0;           // steps asked for one at a time so far (up to SINGLE_STEPS)
     cudaGraphExec_t graph = nullptr;
     int graph_kernels = 0;
@@ -418,6 +421,8 @@ static int upload_run( zpic_sim * s ) {
     return ZPIC_OK;
 }
 
+static int filter_npass( const zpic_sim * s );
+
 // Build the work lists for a set of simulations (one sim, or a batch).
 static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunks_override = 0 ) {
     P.release();
@@ -434,7 +439,7 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
     P.jacc = -1;
     P.tile_n = -1;
     P.needs_bc_or_filter = false;
-    P.sum_in_yee = true;
+    P.sum_in_yee = true; P.filter_in_one = true;
     uint64_t total_tiles = 0; double nominal = 0; int per_sm = 4;
     for ( auto * s : sims ) {
         per_sm = std::min( per_sm, ctas_per_sm( s ) );
@@ -465,6 +470,7 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
             if ( s->emf_bc[k] > ZPIC_EMF_BC_PERIODIC || s->cur_bc[k] > ZPIC_CURRENT_BC_PERIODIC ) P.needs_bc_or_filter = true;
         if ( s->ftype != ZPIC_FILTER_NONE || s->emf_mw.active ) P.needs_bc_or_filter = true;
         if ( s->ftype != ZPIC_FILTER_NONE || s->nxx < 3 || s->nxy < 3 ) P.sum_in_yee = false;
+        if ( !filter_smem_bytes( s->run.extx, s->run.exty, s->fdir, filter_npass( s ) ) ) P.filter_in_one = false;
         for ( int k = 0; k < 4; k++ ) if ( s->cur_bc[k] > ZPIC_CURRENT_BC_PERIODIC ) P.sum_in_yee = false;
     }
     for ( size_t r = 0; r < sims.size(); r++ ) {
@@ -607,8 +613,28 @@ static int run_sort( Plan & P, cudaStream_t st, int use_extra ) {
     return ZPIC_OK;
 }
 
-// Current::advance device part for every run of the plan (current.cpp:227-246)
-static int run_current( Plan & P, cudaStream_t st ) {
+// The 3-point passes of a run's filter (filter.h:22-86): a v[-1] + b v[0] + a v[+1] each.
+static void filter_passes( const zpic_sim * s, std::vector<float> & a, std::vector<float> & b ) {
+    const unsigned order = s->forder > 0 ? s->forder : 1;
+    a.assign( order, 0.25f ); b.assign( order, 0.5f );
+    if ( s->ftype == ZPIC_FILTER_COMPENSATED ) {
+        const float ca = -1.0f;
+        const float cb = ( 4.0 + 2.0 * order ) / order;
+        const float norm = 2 * ca + cb;
+        a.push_back( ca / norm ); b.push_back( cb / norm );
+    }
+}
+
+// Passes of the filter, capped (the order is the caller's, any number).
+static int filter_npass( const zpic_sim * s ) {
+    return s->ftype == ZPIC_FILTER_NONE ? 0 : (int) std::min<unsigned>( s->forder, 1000 ) + ( s->ftype == ZPIC_FILTER_COMPENSATED );
+}
+
+// Current::advance device part for every run of the plan (current.cpp:227-246).
+// In a whole step a plan whose runs all have filters that one kernel can take
+// (filter_in_one) leaves the filtered current in Jdep, for the field solve to
+// read and to keep in J; else the passes run one by one on J.
+static int run_current( Plan & P, cudaStream_t st, bool in_step = false ) {
     {
         PhaseScope ps( prof_sim( P ), st, PH_CURRENT, 1 );
         DEV( launch_current_gc( st, P.tile_items_d, P.n_tiles, P.runs_d, P.max_cells ) );
@@ -625,28 +651,26 @@ static int run_current( Plan & P, cudaStream_t st ) {
             DEV( launch_cur_bc( st, P.runs_d, (int) r, 1, 2 * s->ntx * s->run.extx ) );
         }
     }
-    // filters (filter.h:22-86): run-specific, launched over all tiles of the plan only when uniform
+    // filters: run-specific
+    int first = 0;
     for ( size_t r = 0; r < P.sims.size(); r++ ) {
         zpic_sim * s = P.sims[r];
-        if ( s->ftype == ZPIC_FILTER_NONE ) continue;
-        const unsigned order = s->forder > 0 ? s->forder : 1;
-        // tile items of this run only
-        int first = 0;
-        for ( size_t q = 0; q < r; q++ ) first += P.sims[q]->ntx * P.sims[q]->nty;
-        const int nt = s->ntx * s->nty;
         const TileItem * items = P.tile_items_d + first;
-        auto pass = [&]( float a, float b, float c ) -> int {
+        const int nt = s->ntx * s->nty;
+        first += nt;
+        if ( s->ftype == ZPIC_FILTER_NONE ) continue;
+        std::vector<float> a, b;
+        filter_passes( s, a, b );
+        if ( in_step && P.filter_in_one ) {
+            PhaseScope ps( prof_sim( P ), st, PH_CURRENT, 1 );
+            DEV( launch_filter( st, items, nt, P.runs_d, s->fdir, (int) a.size(), a.data(), b.data(),
+                                filter_smem_bytes( s->run.extx, s->run.exty, s->fdir, (int) a.size() ) ) );
+            continue;
+        }
+        for ( size_t i = 0; i < a.size(); i++ ) {
             PhaseScope ps( prof_sim( P ), st, PH_CURRENT, 2 );
-            DEV( launch_kernel3( st, items, nt, P.runs_d, 2, s->fdir, a, b, c, P.max_tile_vol ) );
+            DEV( launch_kernel3( st, items, nt, P.runs_d, 2, s->fdir, a[i], b[i], a[i], P.max_tile_vol ) );
             DEV( launch_cur_gc( st, items, nt, P.runs_d, s->fdir ? 2 : 1, P.max_guard ) );
-            return ZPIC_OK;
-        };
-        for ( unsigned i = 0; i < order; i++ ) TRY( pass( 0.25f, 0.5f, 0.25f ) );
-        if ( s->ftype == ZPIC_FILTER_COMPENSATED ) {
-            const float a = -1.0f;
-            const float b = ( 4.0 + 2.0 * order ) / order;
-            const float norm = 2 * a + b;
-            TRY( pass( a / norm, b / norm, a / norm ) );
         }
     }
     return ZPIC_OK;
@@ -697,8 +721,8 @@ static int run_shift( Plan & P, cudaStream_t st, int r ) {
 // sum (3x3 cells).
 static int run_current_fields( Plan & P, cudaStream_t st, bool with_shift ) {
     if ( P.sum_in_yee ) return run_fields( P, st, 3, 1, with_shift );
-    TRY( run_current( P, st ) );
-    return run_fields( P, st, 1, 1, with_shift );
+    TRY( run_current( P, st, true ) );
+    return run_fields( P, st, P.filter_in_one ? 4 : 1, 1, with_shift );
 }
 
 static int ensure_plan( zpic_sim * s ) {
@@ -1783,6 +1807,7 @@ int zpic_b200_current_set_filter( zpic_sim * s, int32_t type, int32_t dir, uint3
     if ( type < 0 || type > 2 ) return fail( ZPIC_E_INVALID, "invalid filter type" );
     s->ftype = type; s->fdir = dir ? 1 : 0; s->forder = order > 0 ? order : 1;   // filter.h:35
     s->plan.built = false;
+    s->layout_gen++;                // a batch's plan depends on its runs' filters
     return ZPIC_OK;
 }
 

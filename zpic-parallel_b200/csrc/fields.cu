@@ -296,7 +296,8 @@ __device__ __forceinline__ void yee_e_smem( float * E, const float * B, const fl
 }
 
 // J: where the current comes from.  J_NONE, J_FINAL (R.J), J_RAW (R.Jdep as it
-// is), or J_SUM: the raw deposits of this tile and its neighbours are summed
+// is), J_KEEP (R.Jdep, which holds the filtered current, stored to R.J as well),
+// or J_SUM: the raw deposits of this tile and its neighbours are summed
 // here, into shared memory for the solver and into R.J (guard cells included)
 // for whoever reads the current -- one kernel and one read of J less than a
 // separate sum (Current::advance, current.cpp:227-233).  For tiles of at least
@@ -304,7 +305,7 @@ __device__ __forceinline__ void yee_e_smem( float * E, const float * B, const fl
 // per axis, (own + x neighbour) + (y neighbour + diagonal), and these
 // two-term sums are the same floats whichever tile evaluates them.  The
 // neighbours' values are loaded before the wait for the tile's own copies.
-enum { J_NONE = 0, J_FINAL = 1, J_RAW = 2, J_SUM = 3 };
+enum { J_NONE = 0, J_FINAL = 1, J_RAW = 2, J_SUM = 3, J_KEEP = 4 };
 
 template < int TN, int JSRC >
 __global__ void __launch_bounds__( YEE_THREADS )
@@ -386,7 +387,7 @@ k_yee( const TileItem * __restrict__ items, const RunDev * __restrict__ runs, in
         }
     }
     __syncthreads();
-    if ( JSRC == J_SUM && threadIdx.x == 0 ) {
+    if ( ( JSRC == J_SUM || JSRC == J_KEEP ) && threadIdx.x == 0 ) {
         fence_proxy_async_smem();
         bulk_s2g( R.J + toff, sJ, bytes );
         bulk_commit();
@@ -394,7 +395,7 @@ k_yee( const TileItem * __restrict__ items, const RunDev * __restrict__ runs, in
     yee_e_smem<TN>( E0, B0, J0, sh, R.dtx, R.dty, R.dt, JSRC != J_NONE );
     __syncthreads();
     yee_b_smem<TN>( E0, B0, sh, R.dtx2, R.dty2 );
-    if ( shift_out && JSRC == J_SUM && threadIdx.x == 0 ) bulk_wait_read_all();      // the shifted E takes J's place
+    if ( shift_out && ( JSRC == J_SUM || JSRC == J_KEEP ) && threadIdx.x == 0 ) bulk_wait_read_all();      // the shifted E takes J's place
     __syncthreads();
 
     const float * outE = sE, * outB = sB;
@@ -635,6 +636,76 @@ k_kernel3( const TileItem * __restrict__ items, const RunDev * __restrict__ runs
     }
 }
 
+// All passes of a run's current filter at once (filter.h:22-86: 3-point passes
+// along one axis, each followed by the guard-cell refresh along it), R.J ->
+// R.Jdep.  A CTA filters one tile: it takes the tile's block and `npass` more
+// columns (rows) of its neighbours' interiors, and every pass leaves one
+// column fewer at each end, so that after the last one the block with its
+// guard cells is what the refreshed passes give, bit for bit.  Where there is
+// no neighbour the guard cells are constants, as there.  The passes one by one
+// took two kernels each of 5 us on a small grid (256x64, three passes: 31 us),
+// a chain that the step waited for.
+constexpr int FILTER_THREADS = 256, FILTER_PASSES = 8;
+struct FilterSpec { int diry, npass; float a[FILTER_PASSES], b[FILTER_PASSES]; };      // a v[-1] + b v[0] + a v[+1]
+
+__global__ void __launch_bounds__( FILTER_THREADS )
+k_filter( const TileItem * __restrict__ items, const RunDev * __restrict__ runs, FilterSpec f )
+{
+    extern __shared__ float sA[];
+    const TileItem it = items[ blockIdx.x ];
+    const RunDev & R = runs[ it.run ];
+    const int tx = it.tile % R.ntx, ty = it.tile / R.ntx, h = f.npass;
+    // u runs along the filter, v across: element (u, v) of the wide block
+    const int nu = f.diry ? R.nxy : R.nxx, ne = f.diry ? R.exty : R.extx, nv = f.diry ? R.extx : R.exty;
+    const int w = ne + 2 * h, n = w * nv;
+    const int su = f.diry ? R.extx : 1, sv = f.diry ? 1 : R.extx;       // strides in the tile block
+    const int tl = f.diry ? nbr( ty - 1, R.nty, R.cur_pery ) : nbr( tx - 1, R.ntx, R.cur_perx );
+    const int tr = f.diry ? nbr( ty + 1, R.nty, R.cur_pery ) : nbr( tx + 1, R.ntx, R.cur_perx );
+    const size_t tile = (size_t) R.tile_vol * 3;
+    const float * own = R.J + it.tile * tile;
+    const float * left = tl < 0 ? nullptr : R.J + ( f.diry ? tl * R.ntx + tx : ty * R.ntx + tl ) * tile;
+    const float * right = tr < 0 ? nullptr : R.J + ( f.diry ? tr * R.ntx + tx : ty * R.ntx + tr ) * tile;
+    float * cur = sA, * nxt = sA + 3 * n;
+    for ( int q = threadIdx.x; q < n; q += FILTER_THREADS ) {
+        // consecutive threads along x in either direction
+        const int v = f.diry ? q % nv : q / w, u = ( f.diry ? q / nv : q % w ) - h;     // u: index in the tile block
+        const float * src = own;
+        int uu = u;
+        if ( u < 0 ) { src = left; uu = u + nu; }
+        else if ( u >= ne ) { src = right; uu = u - nu; }
+        float x0 = 0.f, x1 = 0.f, x2 = 0.f;
+        if ( src ) {
+            const float * p = src + 3 * ( uu * su + v * sv );
+            x0 = p[0]; x1 = p[1]; x2 = p[2];
+        }
+        const int k = 3 * ( f.diry ? ( u + h ) * nv + v : v * w + u + h );
+        cur[k] = x0; cur[k + 1] = x1; cur[k + 2] = x2;
+        nxt[k] = x0; nxt[k + 1] = x1; nxt[k + 2] = x2;
+    }
+    __syncthreads();
+    const int d = 3 * ( f.diry ? nv : 1 );                              // one step along the filter, in floats
+    for ( int p = 0; p < h; p++ ) {
+        const int lo = left ? p + 1 - h : GL, hi = right ? ne + h - 1 - p : GL + nu;   // [lo, hi) in the tile block
+        const float a = f.a[p], b = f.b[p];
+        const int m = ( hi - lo ) * nv;
+        for ( int q = threadIdx.x; q < m; q += FILTER_THREADS ) {
+            const int v = f.diry ? q % nv : q / ( hi - lo ), u = lo + ( f.diry ? q / nv : q % ( hi - lo ) );
+            const int k = 3 * ( f.diry ? ( u + h ) * nv + v : v * w + u + h );
+#pragma unroll
+            for ( int j = 0; j < 3; j++ ) nxt[k + j] = cur[k + j - d] * a + cur[k + j] * b + cur[k + j + d] * a;
+        }
+        __syncthreads();
+        float * t = cur; cur = nxt; nxt = t;
+    }
+    float * out = R.Jdep + it.tile * tile;
+    for ( int q = threadIdx.x; q < ne * nv; q += FILTER_THREADS ) {
+        const int i = q % R.extx, j = q / R.extx;
+        const int u = f.diry ? j : i, v = f.diry ? i : j;
+        const int k = 3 * ( f.diry ? ( u + h ) * nv + v : v * w + u + h );
+        out[3 * q] = cur[k]; out[3 * q + 1] = cur[k + 1]; out[3 * q + 2] = cur[k + 2];
+    }
+}
+
 // grid::x_shift_left(1) data motion on E and B (grid.h:455-485); the x guard
 // refresh follows as a separate k_emf_gc( axes = 1 ) launch.  Both fields'
 // tile blocks are staged in shared memory with 16-byte loads in one pass
@@ -775,12 +846,13 @@ cudaError_t launch_cur_gc( cudaStream_t st, const TileItem * items, int n, const
     if ( n > 0 ) k_cur_gc<<< gc_blocks( n, per ), GC_THREADS, 0, st >>>( items, n, per, runs, axes );
     return cudaGetLastError();
 }
-// jsrc: 0 no current, 1 R.J, 2 raw deposits, 3 raw deposits summed over the tiles into R.J
+// jsrc: 0 no current, 1 R.J, 2 raw deposits, 3 raw deposits summed over the tiles into R.J, 4 filtered current in
+// the raw deposits' place, kept in R.J
 cudaError_t launch_yee( cudaStream_t st, const TileItem * items, int n, const RunDev * runs, int jsrc, int max_tile_vol,
                         int shift_out, int tile_n ) {
     typedef void ( *fn )( const TileItem *, const RunDev *, int );
-    static const fn f16[4] = { k_yee< 16, 0 >, k_yee< 16, 1 >, k_yee< 16, 2 >, k_yee< 16, 3 > };
-    static const fn f0[4] = { k_yee< 0, 0 >, k_yee< 0, 1 >, k_yee< 0, 2 >, k_yee< 0, 3 > };
+    static const fn f16[5] = { k_yee< 16, 0 >, k_yee< 16, 1 >, k_yee< 16, 2 >, k_yee< 16, 3 >, k_yee< 16, 4 > };
+    static const fn f0[5] = { k_yee< 0, 0 >, k_yee< 0, 1 >, k_yee< 0, 2 >, k_yee< 0, 3 >, k_yee< 0, 4 > };
     const fn f = ( tile_n == 16 ? f16 : f0 )[ jsrc ];
     const size_t smem = yee_smem_bytes( max_tile_vol );
     if ( smem > 48 * 1024 ) cudaFuncSetAttribute( (const void *) f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem );
@@ -800,6 +872,23 @@ cudaError_t launch_kernel3( cudaStream_t st, const TileItem * items, int n, cons
     const size_t smem = (size_t) 3 * max_tile_vol * sizeof( float );
     if ( smem > 48 * 1024 ) cudaFuncSetAttribute( (const void *) k_kernel3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem );
     if ( n > 0 ) k_kernel3<<< n, 128, smem, st >>>( items, runs, which, diry, a, b, c );
+    return cudaGetLastError();
+}
+// Shared memory of k_filter for tiles of extx x exty cells, 0 when it cannot
+// take them: the passes must stay within the neighbours' interiors.
+size_t filter_smem_bytes( int extx, int exty, int diry, int npass ) {
+    const int nu = ( diry ? exty : extx ) - GL - GU;
+    if ( npass < 1 || npass > FILTER_PASSES || npass > nu - GU ) return 0;
+    const size_t b = 6 * sizeof( float ) * (size_t) ( ( diry ? exty : extx ) + 2 * npass ) * ( diry ? extx : exty );
+    return b <= 200 * 1024 ? b : 0;
+}
+cudaError_t launch_filter( cudaStream_t st, const TileItem * items, int n, const RunDev * runs, int diry, int npass,
+                           const float * a, const float * b, size_t smem ) {
+    FilterSpec f{};
+    f.diry = diry; f.npass = npass;
+    for ( int k = 0; k < npass; k++ ) { f.a[k] = a[k]; f.b[k] = b[k]; }
+    if ( smem > 48 * 1024 ) cudaFuncSetAttribute( (const void *) k_filter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem );
+    if ( n > 0 ) k_filter<<< n, FILTER_THREADS, smem, st >>>( items, runs, f );
     return cudaGetLastError();
 }
 cudaError_t launch_shift_left( cudaStream_t st, const TileItem * items, int n, const RunDev * runs, int max_tile_vol ) {
