@@ -25,9 +25,10 @@
 namespace zb {
 struct TileItem { int run; int tile; };
 size_t particle_smem_bytes( int tile_vol, int jacc );
+int particle_ctas_per_sm( int tile_vol, int jacc );
 size_t yee_smem_bytes( int tile_vol );
 cudaError_t launch_particles( cudaStream_t, int, int, int, const Item *, int, const SpDev *, const RunDev *, const int *,
-                              int, int, int );
+                              int, int, int, double );
 cudaError_t launch_sort( cudaStream_t, const Item *, int, const SegItem *, int, const SpDev *, const RunDev *, int, int *, int, long long, int );
 cudaError_t launch_inject( cudaStream_t, int, int, int, int, int, const SpDev *, const RunDev *, const InjRule &, int );
 cudaError_t launch_inj_dyn( cudaStream_t, float *, unsigned *, int, float, float, float, double );
@@ -130,6 +131,20 @@ constexpr int REORDER_AUTO_STEPS = 50;
 // ---------------------------------------------------------------------------
 // species
 // ---------------------------------------------------------------------------
+// The six arrays of a particle buffer, one allocation: array k starts k *
+// stride bytes after the first (256-byte aligned), so that a kernel reaches
+// all of them from one pointer.
+static int alloc_arrays( PartArrays & a, size_t n ) {
+    a = PartArrays{};
+    const size_t m = ( std::max<size_t>( n, 1 ) + 63 ) & ~(size_t) 63;
+    TRY( dalloc( &a.cell, 6 * m ) );
+    a.stride = m * sizeof( float );
+    float * f = reinterpret_cast<float *>( a.cell );
+    a.xx = f + m; a.xy = f + 2 * m; a.ux = f + 3 * m; a.uy = f + 4 * m; a.uz = f + 5 * m;
+    return ZPIC_OK;
+}
+static void free_arrays( PartArrays & a ) { dfree( a.cell ); a = PartArrays{}; }
+
 struct HSpecies {
     std::string name;
     float m_q = -1; uint32_t ppc[2] = { 1, 1 };
@@ -153,8 +168,7 @@ struct HSpecies {
     unsigned * mw_nmove_d = nullptr;   // device copy of the window's move count
 
     void free_all() {
-        PartArrays * arrs[2] = { &d.A, &d.B };
-        for ( auto * a : arrs ) { dfree( a->cell ); dfree( a->xx ); dfree( a->xy ); dfree( a->ux ); dfree( a->uy ); dfree( a->uz ); }
+        free_arrays( d.A ); free_arrays( d.B );
         dfree( d.np ); dfree( d.off ); dfree( d.cap ); dfree( d.nidx ); dfree( d.idx );
         dfree( d.aux ); dfree( d.aux2 ); dfree( d.in_cnt ); dfree( d.stage_cnt );
         dfree( d.cnt ); dfree( d.base ); dfree( d.hs ); dfree( d.overflow ); dfree( d.reloc ); dfree( d.pool );
@@ -163,12 +177,6 @@ struct HSpecies {
         dfree( d.energy ); dfree( d.nmove ); dfree( inj_dyn ); dfree( mw_nmove_d );
     }
 };
-
-static int alloc_arrays( PartArrays & a, size_t n ) {
-    TRY( dalloc( &a.cell, n ) ); TRY( dalloc( &a.xx, n ) ); TRY( dalloc( &a.xy, n ) );
-    TRY( dalloc( &a.ux, n ) ); TRY( dalloc( &a.uy, n ) ); TRY( dalloc( &a.uz, n ) );
-    return ZPIC_OK;
-}
 
 // ---------------------------------------------------------------------------
 // plan: device work lists over a set of simulations
@@ -191,6 +199,7 @@ struct Plan {
     Item * spk1_d = nullptr;
     std::vector<int> sp_k1_off, sp_k1_n, sp_sort_off, sp_sort_n, sp_seg_off, sp_seg_n;
     TileItem * tile_items_d = nullptr; int n_tiles = 0;
+    double per_cta = 0;             // particles per CTA of the particle kernel, in the fullest tiles of a full plasma
     int max_tile_vol = 0;
     int max_cells = 0, max_guard = 0;   // cells and guard cells of the largest tile
     int max_nxy = 0;                // tile rows (cells in y) of the tallest tile
@@ -367,7 +376,7 @@ struct Workspace {
 // launch would take: its waves of resident CTAs (per_sm of them on an SM),
 // each CTA with its fixed part (set-up, field staging, write-back of the tile
 // current) and its particles, plus the cost of every CTA launched.  Measured:
-// 10.3 ns per particle in a full wave, 5 us fixed, 8.2 ns per CTA.  Small runs
+// 15.6 ps per particle with all slots busy, 5 us fixed, 8.2 ns per CTA.  Small runs
 // get one full wave rather than two and a bit (128x128 Weibel set-up, 4 CTAs
 // per tile instead of 10: 41 against 47 us per step while it is uniform; 64x64
 // cells 33 -> 26 us), few large tiles several (512 tiles of 32x32 cells, 6
@@ -376,22 +385,23 @@ static int auto_chunks( uint64_t ntiles, double particles_per_tile, int per_sm, 
     if ( opt > 0 ) return opt;
     int dev = 0; cudaGetDevice( &dev );
     int sms = 148; cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
+    // with enough tiles one CTA each, whose current does not depend on the order
+    // of its sums: the same from run to run
+    if ( ntiles >= (uint64_t) sms * 8 ) return 1;
     const double slots = (double) sms * per_sm;
     int best = 1; double best_us = 0;
     for ( int c = 1; c <= 64; c++ ) {
         const double ctas = (double) ntiles * c;
-        const double us = std::ceil( ctas / slots ) * ( 0.0103 * particles_per_tile / c + 5.0 ) + 0.0082 * ctas;
+        const double us = std::ceil( ctas / slots ) * ( 15.6e-6 * slots * particles_per_tile / c + 5.0 ) + 0.0082 * ctas;
         if ( c == 1 || us < best_us ) { best = c; best_us = us; }
     }
     return best;
 }
 
 // Particles per tile of a full plasma, and CTAs of the particle kernel per SM
-// (64 registers a thread allow four; large tiles fewer by their shared memory).
+// (six of 128 threads by their registers; large tiles fewer by their shared memory).
 static double nominal_per_tile( const zpic_sim * s, const HSpecies * h ) { return (double) h->ppc[0] * h->ppc[1] * s->nxx * s->nxy; }
-static int ctas_per_sm( const zpic_sim * s ) {
-    return std::max( 1, std::min( 4, (int) ( 227 * 1024 / ( particle_smem_bytes( s->run.tile_vol, s->jacc ) + 1024 ) ) ) );
-}
+static int ctas_per_sm( const zpic_sim * s ) { return particle_ctas_per_sm( s->run.tile_vol, s->jacc ); }
 
 // CTAs per tile of the particle kernel ("chunks" option): n > 0 for every
 // tile; 0, the automatic choice, for every tile; -1 balanced: a tile of
@@ -434,7 +444,7 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
     std::vector<TileItem> tiles;
     P.sps_h.clear(); P.sp_sim.clear(); P.sp_local.clear();
     P.sp_k1_off.clear(); P.sp_k1_n.clear(); P.sp_sort_off.clear(); P.sp_sort_n.clear(); P.sp_seg_off.clear(); P.sp_seg_n.clear();
-    P.max_tile_vol = 0;
+    P.max_tile_vol = 0; P.per_cta = 0;
     P.max_cells = 0; P.max_guard = 0; P.max_tile_cells = 0; P.max_nxy = 0;
     P.reorder_every = 0; P.reorder_count = 0;
     P.jacc = -1;
@@ -480,6 +490,7 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
             HSpecies * sp = s->species[k];
             SpDev d = sp->d;
             if ( batch_chunks ) { d.nchunk = batch_chunks; d.chunk_target = 0; }
+            P.per_cta = std::max( P.per_cta, nominal_per_tile( s, sp ) / d.nchunk );
             d.run = (int) r;
             const int gi = (int) P.sps_h.size();
             P.sps_h.push_back( d );
@@ -599,7 +610,7 @@ static int run_particles( Plan & P, cudaStream_t st, int push, int move, const i
         if ( P.n_k1[p] == 0 ) continue;
         PhaseScope ps( prof_sim( P ), st, PH_PARTICLES, 1 );
         DEV( launch_particles( st, push ? p + 1 : 0, move, 1, P.k1_items_d[p], P.n_k1[p], P.sps_d, P.runs_d, shifts, P.max_tile_vol,
-                              P.jacc, P.tile_n ) );
+                              P.jacc, P.tile_n, P.per_cta ) );
     }
     return ZPIC_OK;
 }
@@ -1073,8 +1084,7 @@ static int species_grow( zpic_sim * s, HSpecies * h, uint64_t new_max ) {
     if ( rc == ZPIC_OK ) rc = dalloc( &aux, new_max );
     if ( rc == ZPIC_OK ) rc = dalloc( &aux2, new_max );
     if ( rc != ZPIC_OK ) {
-        PartArrays * na[2] = { &A, &B };
-        for ( auto * a : na ) { dfree( a->cell ); dfree( a->xx ); dfree( a->xy ); dfree( a->ux ); dfree( a->uy ); dfree( a->uz ); }
+        free_arrays( A ); free_arrays( B );
         dfree( idx ); dfree( aux ); dfree( aux2 );
         return rc;
     }
@@ -1090,8 +1100,7 @@ static int species_grow( zpic_sim * s, HSpecies * h, uint64_t new_max ) {
     }
     CK( cudaMemcpyAsync( idx, d.idx, old * sizeof( int ), cudaMemcpyDeviceToDevice, s->stream ) );
     CK( cudaStreamSynchronize( s->stream ) );
-    PartArrays * olds[2] = { &d.A, &d.B };
-    for ( auto * a : olds ) { dfree( a->cell ); dfree( a->xx ); dfree( a->xy ); dfree( a->ux ); dfree( a->uy ); dfree( a->uz ); }
+    free_arrays( d.A ); free_arrays( d.B );
     dfree( d.idx ); dfree( d.aux ); dfree( d.aux2 );
     d.A = A; d.B = B; d.idx = idx; d.aux = aux; d.aux2 = aux2;
     d.max_part = (int) new_max;
@@ -1186,7 +1195,7 @@ static int species_kernel( zpic_sim * s, int sp, int push, int move, const int *
         PhaseScope ps( s, s->stream, PH_PARTICLES, 1 );
         DEV( launch_particles( s->stream, push ? 1 + h->push_type : 0, move, move ? 1 : 0,
                               P.spk1_d + P.sp_k1_off[sp], P.sp_k1_n[sp], P.sps_d, P.runs_d, shifts, P.max_tile_vol,
-                              P.jacc, P.tile_n ) );
+                              P.jacc, P.tile_n, P.per_cta ) );
     }
     if ( move ) { h->sort_pending = true; h->counters_dirty = true; }
     if ( push ) h->energy_items = h->ntiles * P.sps_h[sp].nchunk;
@@ -1204,7 +1213,7 @@ static int species_sort( zpic_sim * s, int sp, int use_extra ) {
         DEV( cudaMemsetAsync( h->d.nidx, 0, h->ntiles * sizeof( int ), s->stream ) );
         PhaseScope ps( s, s->stream, PH_SORT, 1 );
         DEV( launch_particles( s->stream, 0, 0, 1, P.spk1_d + P.sp_k1_off[sp], P.sp_k1_n[sp], P.sps_d, P.runs_d,
-                              nullptr, P.max_tile_vol, 0, 0 ) );
+                              nullptr, P.max_tile_vol, 0, 0, P.per_cta ) );
     }
     {
         PhaseScope ps( s, s->stream, PH_SORT, 3 );

@@ -115,30 +115,176 @@ __device__ __forceinline__ void dudt_boris_euler( float alpha, float ex, float e
     uz = __fmaf_rn( r13, utx, __fmaf_rn( r23, uty, r33 * utz ) ) + ez;
 }
 
+// ---------------------------------------------------------------------------
+// Two particles at a time
+//
+// A thread pushes, moves and deposits its two particles together, their FP32
+// values in the two halves of 64-bit registers, with sm_100's packed
+// instructions (add, mul and fma .f32x2): one instruction slot for two
+// particles, each half rounded as the scalar instruction rounds it.  The
+// particle kernel is bound by instruction issue.
+// ---------------------------------------------------------------------------
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 pack2( float a, float b ) { F2 r; asm( "mov.b64 %0, {%1, %2};" : "=l"( r.v ) : "f"( a ), "f"( b ) ); return r; }
+__device__ __forceinline__ F2 both( float a ) { return pack2( a, a ); }
+__device__ __forceinline__ void unpack2( F2 x, float & a, float & b ) { asm( "mov.b64 {%0, %1}, %2;" : "=f"( a ), "=f"( b ) : "l"( x.v ) ); }
+__device__ __forceinline__ F2 operator+( F2 a, F2 b ) { F2 r; asm( "add.rn.f32x2 %0, %1, %2;" : "=l"( r.v ) : "l"( a.v ), "l"( b.v ) ); return r; }
+__device__ __forceinline__ F2 operator-( F2 a, F2 b ) { F2 r; asm( "sub.rn.f32x2 %0, %1, %2;" : "=l"( r.v ) : "l"( a.v ), "l"( b.v ) ); return r; }
+__device__ __forceinline__ F2 operator*( F2 a, F2 b ) { F2 r; asm( "mul.rn.f32x2 %0, %1, %2;" : "=l"( r.v ) : "l"( a.v ), "l"( b.v ) ); return r; }
+__device__ __forceinline__ F2 fma2( F2 a, F2 b, F2 c ) { F2 r; asm( "fma.rn.f32x2 %0, %1, %2, %3;" : "=l"( r.v ) : "l"( a.v ), "l"( b.v ), "l"( c.v ) ); return r; }
+// The product that a sum takes up.  The assembler contracts a packed product and
+// the sum that uses it into one fused operation, whatever it is told about
+// contraction, and the reference rounds in between: nz is {-0, -0} from memory,
+// so that it cannot know that adding it changes nothing.
+__device__ __forceinline__ F2 mul2( F2 a, F2 b, F2 nz ) { return fma2( a, b, nz ); }
+// (folded into the consuming instruction's operand)
+__device__ __forceinline__ F2 neg2( F2 a ) { float x, y; unpack2( a, x, y ); return pack2( -x, -y ); }
+
+// Correctly rounded square root, reciprocal and quotient for arguments in
+// [1, QLIM): an approximation by the special-function unit, then one Newton
+// step on the exact remainder that fma gives (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34, 1990).  The same floats as the IEEE operations, without their tests
+// of the argument's range at each call: every float of [1, 2^96) was compared
+// for the root and the reciprocal, every one of [1, 2^12) with 64 numerators
+// for the quotient; the theorem behind the last step holds for all numerators
+// whose quotient and remainder are normal numbers.
+constexpr float QLIM = 7.9e28f;             // about 2^96
+__device__ __forceinline__ F2 sqrt2( F2 x ) {
+    float a, b, ra, rb;
+    unpack2( x, a, b );
+    asm( "rsqrt.approx.ftz.f32 %0, %1;" : "=f"( ra ) : "f"( a ) );
+    asm( "rsqrt.approx.ftz.f32 %0, %1;" : "=f"( rb ) : "f"( b ) );
+    const F2 r = pack2( ra, rb );
+    const F2 g = x * r;
+    return fma2( fma2( g, neg2( g ), x ), r * both( 0.5f ), g );
+}
+__device__ __forceinline__ F2 recip2( F2 d ) {
+    float a, b, ra, rb;
+    unpack2( d, a, b );
+    asm( "rcp.approx.ftz.f32 %0, %1;" : "=f"( ra ) : "f"( a ) );
+    asm( "rcp.approx.ftz.f32 %0, %1;" : "=f"( rb ) : "f"( b ) );
+    const F2 r = pack2( ra, rb );
+    return fma2( r, fma2( d, neg2( r ), both( 1.0f ) ), r );
+}
+// a / d, with y = recip2( d )
+__device__ __forceinline__ F2 quot2( F2 a, F2 d, F2 y ) {
+    const F2 q = a * y;
+    return fma2( fma2( d, neg2( q ), a ), y, q );
+}
+
+// interpolate_fld for two particles: cells (ia, ja), (ib, jb)
+__device__ __forceinline__ void interpolate_fld2( const float * __restrict__ E, const float * __restrict__ B, int ys,
+                                                  int ia, int ja, int ib, int jb, float xa, float ya, float xb, float yb,
+                                                  F2 nz, F2 & ex, F2 & ey, F2 & ez, F2 & bx, F2 & by, F2 & bz ) {
+    const F2 x = pack2( xa, xb ), y = pack2( ya, yb ), half = both( 0.5f ), one = both( 1.0f );
+    const F2 s0x = half - x, s1x = half + x, s0y = half - y, s1y = half + y;
+    const F2 hx = pack2( xa < 0 ? 1.0f : 0.0f, xb < 0 ? 1.0f : 0.0f ), hy = pack2( ya < 0 ? 1.0f : 0.0f, yb < 0 ? 1.0f : 0.0f );
+    const F2 s0xh = ( one - hx ) - x, s1xh = hx + x, s0yh = ( one - hy ) - y, s1yh = hy + y;
+    const int s3 = 3 * ys;
+    const int a = 3 * ( ia + ys * ja ), b = 3 * ( ib + ys * jb );
+    const int ahx = xa < 0 ? 3 : 0, ahy = ya < 0 ? s3 : 0, bhx = xb < 0 ? 3 : 0, bhy = yb < 0 ? s3 : 0;
+#define FP( F, k, oa, ob ) pack2( F[ ( oa ) + ( k ) ], F[ ( ob ) + ( k ) ] )
+#define ROW( F, k, oa, ob, wx0, wx1 ) ( mul2( FP( F, k, oa, ob ), wx0, nz ) + mul2( FP( F, k, ( oa ) + 3, ( ob ) + 3 ), wx1, nz ) )
+#define C4( F, k, oa, ob, wx0, wx1, wy0, wy1 ) \
+    ( mul2( ROW( F, k, oa, ob, wx0, wx1 ), wy0, nz ) + mul2( ROW( F, k, ( oa ) + s3, ( ob ) + s3, wx0, wx1 ), wy1, nz ) )
+    ex = C4( E, 0, a - ahx, b - bhx, s0xh, s1xh, s0y, s1y );
+    by = C4( B, 1, a - ahx, b - bhx, s0xh, s1xh, s0y, s1y );
+    ey = C4( E, 1, a - ahy, b - bhy, s0x, s1x, s0yh, s1yh );
+    bx = C4( B, 0, a - ahy, b - bhy, s0x, s1x, s0yh, s1yh );
+    ez = C4( E, 2, a, b, s0x, s1x, s0y, s1y );
+    bz = C4( B, 2, a - ahx - ahy, b - bhx - bhy, s0xh, s1xh, s0yh, s1yh );
+#undef C4
+#undef ROW
+#undef FP
+}
+
+// dudt_boris for two particles.  u: in and out; en: the two energy terms.
+// False when a value is out of range of the pair arithmetic (or not a
+// number); u and en are then not to be used.
+__device__ __forceinline__ bool dudt_boris2( F2 al, F2 nz, F2 ex, F2 ey, F2 ez, F2 bx, F2 by, F2 bz,
+                                             F2 & ux, F2 & uy, F2 & uz, F2 & en ) {
+    const F2 one = both( 1.0f );
+    ex = mul2( ex, al, nz ); ey = mul2( ey, al, nz ); ez = mul2( ez, al, nz );
+    F2 utx = ux + ex, uty = uy + ey, utz = uz + ez;
+    const F2 utsq = fma2( utz, utz, fma2( uty, uty, utx * utx ) );
+    const F2 g2 = one + utsq;
+    const F2 gamma = sqrt2( g2 );
+    const F2 g1 = gamma + one;
+    en = quot2( utsq, g1, recip2( g1 ) );
+    const F2 ag = quot2( al, gamma, recip2( gamma ) );
+    bx = bx * ag; by = by * ag; bz = bz * ag;
+    F2 vx = fma2( bz, uty, utx );
+    F2 vy = fma2( bx, utz, uty );
+    F2 vz = fma2( by, utx, utz );
+    vx = fma2( neg2( by ), utz, vx );
+    vy = fma2( neg2( bz ), utx, vy );
+    vz = fma2( neg2( bx ), uty, vz );
+    const F2 d = fma2( bz, bz, fma2( by, by, fma2( bx, bx, one ) ) );
+    const F2 r = recip2( d );
+    const F2 otsq = r + r;
+    bx = bx * otsq; by = by * otsq; bz = bz * otsq;
+    utx = fma2( bz, vy, utx );
+    uty = fma2( bx, vz, uty );
+    utz = fma2( by, vx, utz );
+    utx = fma2( neg2( by ), vz, utx );
+    uty = fma2( neg2( bz ), vx, uty );
+    utz = fma2( neg2( bx ), vy, utz );
+    ux = utx + ex; uy = uty + ey; uz = utz + ez;
+    float ga, gb, da, db;
+    unpack2( g2, ga, gb ); unpack2( d, da, db );
+    return ga < QLIM && gb < QLIM && da < QLIM && db < QLIM;
+}
+
+// rgamma for two particles; false when out of range
+__device__ __forceinline__ bool rgamma2( F2 ux, F2 uy, F2 uz, F2 & rg ) {
+    const F2 g2 = fma2( uz, uz, fma2( uy, uy, fma2( ux, ux, both( 1.0f ) ) ) );
+    rg = recip2( sqrt2( g2 ) );
+    float a, b;
+    unpack2( g2, a, b );
+    return a < QLIM && b < QLIM;
+}
+
+// The push of one particle with the general operations, for the pairs that
+// are out of range of the pair arithmetic: the new momentum and (w) the
+// energy term.
+__device__ __noinline__ float4 push_one( const float * E, const float * B, int ys, int i, int j, float xx, float xy, float alpha,
+                                         float ux, float uy, float uz ) {
+    float ex, ey, ez, bx, by, bz;
+    double en = 0.0;
+    interpolate_fld( E, B, ys, i, j, xx, xy, ex, ey, ez, bx, by, bz );
+    dudt_boris( alpha, ex, ey, ez, bx, by, bz, ux, uy, uz, en );
+    return make_float4( ux, uy, uz, (float) en );
+}
+
 // Accumulation of one current contribution into the shared-memory tile
 // current: FP32 or FP64 atomics, or fixed point.  Fixed point: the
 // contribution arrives already multiplied by js (a power of two that keeps
 // every contribution below 2^31 in magnitude, folded into the charge factors)
-// and is rounded to an integer x; floor(x / 2^16) is added to a hi word and x
-// itself (mod 2^32) to a second word jlo entries later, both with native
-// shared-memory integer atomics.  Integer sums do not depend on the order of
-// the additions; the hi sum cannot overflow and the low parts are recovered
-// exactly for up to 2^16 additions per entry, and the kernel flushes the
-// accumulators before that many.
+// and is rounded to an integer x, which a native shared-memory integer atomic
+// adds to a word (mod 2^32).  The old value it returns tells whether the word,
+// taken as signed, wrapped; then a second atomic counts the wrap in a word jlo
+// entries later, so that word + 2^32 count is the exact sum, whatever the order
+// and the number of additions.  (Two atomics for every contribution -- the
+// upper 16 bits and the whole word -- took twice the wavefronts: 33 instead of
+// 17 of the 82 M of a step of 16.8 M particles in decayed order, 10 % of the
+// kernel's time.  A wrap is rare: |x| / 2^32 of the additions.)
 struct JAcc { float js; int jlo; };
 __device__ __forceinline__ void jadd( float * p, float v, JAcc ) { atomicAdd( p, v ); }
 __device__ __forceinline__ void jadd( double * p, float v, JAcc ) { atomicAdd( p, (double) v ); }
+// x added to the word at p (mod 2^32); -1, 0 or 1 when the word, taken as
+// signed, wrapped
+__device__ __forceinline__ bool wrapped( int o, int x ) {
+    const int n = (int) ( (unsigned) o + (unsigned) x );
+    return ( ( o ^ n ) & ( x ^ n ) ) < 0;
+}
 __device__ __forceinline__ void jadd( int * p, float v, JAcc a ) {
     const int x = __float2int_rn( v );
-    atomicAdd( p, x >> 16 );
-    atomicAdd( reinterpret_cast<unsigned int *>( p + a.jlo ), (unsigned int) x );
+    const int o = atomicAdd( p, x );
+    if ( wrapped( o, x ) ) atomicAdd( p + a.jlo, x < 0 ? -1 : 1 );
 }
-// value of a fixed-point accumulator pair: hi = sum of floor(x / 2^16),
-// full = sum of x mod 2^32, so full - hi * 2^16 (mod 2^32) is the sum of the
-// low 16-bit parts, exact below 2^32 (up to 65537 additions).
-__device__ __forceinline__ double jfix_value( int hi, unsigned int full, double inv ) {
-    const unsigned int lo = full - ( (unsigned int) hi << 16 );
-    return ( (double) hi * 65536.0 + (double) lo ) * inv;
+__device__ __forceinline__ double jfix_value( int w, int c, double inv ) {
+    return ( (double) c * 4294967296.0 + (double) w ) * inv;
 }
 
 // Charge-conserving current of one segment inside one cell (species.cpp:267-310),
@@ -177,6 +323,54 @@ __device__ __forceinline__ void dep_current_seg( int ix, int iy, float x0x, floa
         jadd( Js + s3 + 2, qvz * ( S0x0 * S0y1 + S1x0 * S1y1 + ( S0x0 * S1y1 - S1x0 * S0y1 ) / 2.0f ), ja );
         jadd( Js + s3 + 5, qvz * ( S0x1 * S0y1 + S1x1 * S1y1 + ( S0x1 * S1y1 - S1x1 * S0y1 ) / 2.0f ), ja );
     }
+}
+
+// The eight contributions of dep_current_seg's fixed-point form for two
+// segments: w[0..3] in plane (Jx at (0,0) and (0,1), Jy at (0,0) and (1,0)),
+// w[4..7] out of plane (Jz at (0,0), (1,0), (0,1), (1,1)).
+__device__ __forceinline__ void current_seg2( F2 x0x, F2 x0y, F2 x1x, F2 x1y, F2 hqx, F2 hqy, F2 qvz, F2 w[8] ) {
+    const F2 half = both( 0.5f ), mhalf = both( -0.5f );
+    const F2 S0x0 = half - x0x, S0x1 = half + x0x, S1x0 = half - x1x, S1x1 = half + x1x;
+    const F2 S0y0 = half - x0y, S0y1 = half + x0y, S1y0 = half - x1y, S1y1 = half + x1y;
+    const F2 wl1 = hqx * ( x1x - x0x ), wl2 = hqy * ( x1y - x0y );
+    w[0] = wl1 * ( S0y0 + S1y0 );
+    w[1] = wl1 * ( S0y1 + S1y1 );
+    w[2] = wl2 * ( S0x0 + S1x0 );
+    w[3] = wl2 * ( S0x1 + S1x1 );
+    const F2 qp0 = qvz * fma2( S1y0, half, S0y0 ), qq0 = qvz * fma2( S0y0, mhalf, S1y0 );
+    const F2 qp1 = qvz * fma2( S1y1, half, S0y1 ), qq1 = qvz * fma2( S0y1, mhalf, S1y1 );
+    w[4] = fma2( S0x0, qp0, S1x0 * qq0 );
+    w[5] = fma2( S0x1, qp0, S1x1 * qq0 );
+    w[6] = fma2( S0x0, qp1, S1x0 * qq1 );
+    w[7] = fma2( S0x1, qp1, S1x1 * qq1 );
+}
+// adds one segment's contributions (fixed point) at cell (ix, iy)
+__device__ __forceinline__ void add_seg( int * J, int ix, int iy, int stride, const float w[8], JAcc ja ) {
+    int * Js = J + 3 * ( ix + stride * iy );
+    const int s3 = 3 * stride;
+    const int at[8] = { 0, s3, 1, 3 + 1, 2, 3 + 2, s3 + 2, s3 + 5 };
+    int x[8], o[8];
+#pragma unroll
+    for ( int k = 0; k < 8; k++ ) { x[k] = __float2int_rn( w[k] ); o[k] = atomicAdd( Js + at[k], x[k] ); }
+    int any = 0;
+#pragma unroll
+    for ( int k = 0; k < 8; k++ ) { const int n = (int) ( (unsigned) o[k] + (unsigned) x[k] ); any |= ( o[k] ^ n ) & ( x[k] ^ n ); }
+    if ( any < 0 ) {
+#pragma unroll
+        for ( int k = 0; k < 8; k++ ) if ( wrapped( o[k], x[k] ) ) atomicAdd( Js + at[k] + ja.jlo, x[k] < 0 ? -1 : 1 );
+    }
+}
+// dep_current_seg for two segments, a where da and b where db
+__device__ __forceinline__ void dep_current_seg2( bool da, int ixa, int iya, bool db, int ixb, int iyb,
+                                                  F2 x0x, F2 x0y, F2 x1x, F2 x1y, F2 hqx, F2 hqy, F2 qvz,
+                                                  int * J, int stride, JAcc ja ) {
+    F2 w[8];
+    float wa[8], wb[8];
+    current_seg2( x0x, x0y, x1x, x1y, hqx, hqy, qvz, w );
+#pragma unroll
+    for ( int k = 0; k < 8; k++ ) unpack2( w[k], wa[k], wb[k] );
+    if ( da ) add_seg( J, ixa, iya, stride, wa, ja );
+    if ( db ) add_seg( J, ixb, iyb, stride, wb, ja );
 }
 
 // Split the trajectory of a particle that crosses at least one cell edge into
@@ -230,13 +424,18 @@ __device__ __forceinline__ void deposit_crossing( int ix, int iy, float x0x, flo
             v1y1 -= diy;
         }
     }
-    dep_current_seg( v0x, v0y, v0x0, v0y0, v0x1, v0y1, qnxx, qnxy, v0q, J, stride, ja );
-    dep_current_seg( v1x, v1y, v1x0, v1y0, v1x1, v1y1, qnxx, qnxy, v1q, J, stride, ja );
+    if constexpr ( std::is_same<JT, int>::value ) {
+        dep_current_seg2( true, v0x, v0y, true, v1x, v1y, pack2( v0x0, v1x0 ), pack2( v0y0, v1y0 ), pack2( v0x1, v1x1 ),
+                          pack2( v0y1, v1y1 ), both( qnxx ), both( qnxy ), pack2( v0q, v1q ), J, stride, ja );
+    } else {
+        dep_current_seg( v0x, v0y, v0x0, v0y0, v0x1, v0y1, qnxx, qnxy, v0q, J, stride, ja );
+        dep_current_seg( v1x, v1y, v1x0, v1y0, v1x1, v1y1, qnxx, qnxy, v1q, J, stride, ja );
+    }
     if ( crossx && crossy ) dep_current_seg( v2x, v2y, v2x0, v2y0, v2x1, v2y1, qnxx, qnxy, v2q, J, stride, ja );
 }
 
 // Per-warp ring of cell-crossing particles waiting for their split deposit.
-constexpr int XQ = 64;                      // entries per warp (power of two)
+constexpr int XQ = 96;                      // entries per warp: up to 31 left over and 64 of one iteration
 struct CrossQueue {
     uint32_t cell[XQ];
     float x0x[XQ], x0y[XQ], dx[XQ], dy[XQ], qvz[XQ];
@@ -264,18 +463,33 @@ __device__ __noinline__ void drain_entry( const CrossQueue & Q, int e, float qnx
 // E and B tiles (guard cells included, the contiguous tile_vol block) are
 // staged into shared memory with one bulk asynchronous copy each; the tile
 // current is accumulated in shared memory and added to the raw current buffer
-// with one bulk reduce-add.  Thread t handles particles t and t+256 of each
-// 512-particle block (2 per thread keeps 4 CTAs per SM resident without
-// spills, 35% faster than 4 per thread): every access is a fully coalesced 128 B
-// warp transaction, and consecutive lanes (consecutive particles, which the
-// injection order puts in consecutive cells) spread over the shared-memory
-// banks (about 2-way conflicts; as particles drift between the cells of their
-// tile the order decays towards random cells, about 3.5-way, which the
-// optional in-tile reorder undoes).  Particles that stay in their cell deposit
-// one segment at once; particles that cross a cell edge are queued per warp
-// and split/deposited in full-warp passes, so the split runs on full warps
-// (only a third segment, for the rare double crossings, diverges).
+// with one bulk reduce-add.  A warp takes 64 consecutive particles at a time,
+// a lane the particles `lane` and `lane + 32` of them as a pair (every access a
+// coalesced 128 B warp transaction), and prefetches the lines of its next 64
+// into L1.  Consecutive lanes (consecutive particles, which the injection
+// order puts in consecutive cells) spread over the shared-memory banks (about
+// 2-way conflicts; as particles drift between the cells of their tile the order
+// decays towards random cells, about 3.5-way, which the optional in-tile
+// reorder undoes).  Particles that stay in their cell deposit one segment at
+// once; particles that cross a cell edge are queued per warp and
+// split/deposited in full-warp passes, so the split runs on full warps (only a
+// third segment, for the rare double crossings, diverges).
+//
+// What bounds it: the L1 data pipe (field reads and current atomics) and the
+// latency between them, with 24 warps per SM at 80 registers.  1024^2 cells,
+// 67 M particles, about 40 steps after a reorder: scalar arithmetic with two
+// shared atomics per contribution 1236 us (525 instructions and 156 wavefronts
+// per warp of particles), pairs with one atomic and a counted wrap 1147 us
+// (390 and 132); 4.2 M particles in 4,096 tiles 143 -> 131 us, 35x21-cell
+// tiles with the exact rotation 104 -> 83 us.  64 registers (32 warps) spill:
+// 7 % slower.  Register, bulk-copy and cp.async staging of the next particles
+// instead of the prefetch: 14, 12 and 1 % slower.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void copy_particle( const PartArrays & d, size_t di, const PartArrays & s, size_t si ) {
+    d.cell[di] = s.cell[si]; d.xx[di] = s.xx[si]; d.xy[di] = s.xy[si];
+    d.ux[di] = s.ux[si]; d.uy[di] = s.uy[si]; d.uz[di] = s.uz[si];
+}
+
 // Block-wide exclusive scan of one value per thread; the block total is
 // written to *total (a shared variable) and visible on return.
 template < int NT >
@@ -315,41 +529,42 @@ __device__ __forceinline__ int wrap_tile( int v, int n, int periodic ) {
     return ( v >= 0 && v < n ) ? v : -1;
 }
 
-constexpr int PK_THREADS = 256;
-constexpr int PK_PPT = 2;                   // particles per thread per block iteration
-// Particles between fixed-point flushes: at most 3 additions per particle and
-// accumulator pair, 61,440 < 2^16 per group.  Tiles of 16x16 cells at 8x8
-// particles per cell (16,384 on average) then run without a flush.
-constexpr int FLUSH_PARTICLES = 20480;
-static_assert( FLUSH_PARTICLES % ( PK_PPT * PK_THREADS ) == 0, "flush groups hold whole blocks" );
+constexpr int WP = 64;                      // particles of one warp iteration (a pair per lane)
+constexpr int PK_PPT = 2;
+// CTAs per SM that the registers allow, at 80 a thread.  (7 of 128 threads at
+// 72 spill: 128x128 Weibel set-up 57 -> 56 us per step, but 4096x512 wakefield
+// 534 -> 543 and 24x14-cell tiles 34 -> 36.)
+constexpr int pk_ctas( int threads ) { return 768 / threads; }
 
-// Adds the fixed-point tile current accumulated so far (hi words at acc[0, n),
-// full words at acc[n, 2n)) to the raw current of the tile and clears it.  Out
-// of line: it runs once per FLUSH_PARTICLES particles of a CTA, at most.
-__device__ __noinline__ void jfix_flush( int * acc, int n, float * __restrict__ dst, double inv ) {
-    __syncthreads();
-    unsigned int * full = reinterpret_cast<unsigned int *>( acc ) + n;
-    for ( int i = threadIdx.x; i < n; i += blockDim.x ) {
-        const int h = acc[i];
-        const unsigned int l = full[i];
-        if ( h != 0 || l != 0 ) {
-            atomicAdd( dst + i, (float) jfix_value( h, l, inv ) );
-            acc[i] = 0;
-            full[i] = 0;
-        }
-    }
-    __syncthreads();
+// The species' factors, each in both halves of a pair; read from shared memory
+// where they are used rather than held in registers through the loop.
+struct __align__( 16 ) PairFactors { F2 dt_dx, dt_dy, qnxx, qnxy, alpha, qhalf, nz, pad; };      // nz: {-0, -0} (mul2)
+__device__ __forceinline__ F2 lds2( const F2 & p ) {
+    F2 r;
+    asm volatile( "ld.shared.b64 %0, [%1];" : "=l"( r.v ) : "r"( smem_u32( &p ) ) );
+    return r;
+}
+// two adjacent factors, the first 16-byte aligned
+__device__ __forceinline__ void lds2x2( const F2 & p, F2 & a, F2 & b ) {
+    asm volatile( "ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"( a.v ), "=l"( b.v ) : "r"( smem_u32( &p ) ) );
+}
+__device__ __forceinline__ float lds1( const F2 & p ) {
+    float r;
+    asm volatile( "ld.shared.f32 %0, [%1];" : "=f"( r ) : "r"( smem_u32( &p ) ) );
+    return r;
 }
 
 // JT is the type of the tile current accumulated in shared memory: float
 // (FP32 sums, as the reference), double (FP64 sums) or int (fixed point in
-// two 32-bit words, order-independent); the last two are rounded
-// to FP32 once per cell when the tile is added to the global deposit buffer.
+// a 32-bit word and a count of its wraps, order-independent); the last two are
+// rounded to FP32 once per cell when the tile is added to the global deposit
+// buffer.
 // TN > 0 fixes square TN x TN tiles at compile time, so every shared-memory
 // offset of the interpolation and deposit stencils is an immediate; TN = 0
-// reads the tile shape from the run descriptor.
-template < int PUSH, int MOVE, bool DETECT, typename JT = float, int TN = 0 >
-__global__ void __launch_bounds__( PK_THREADS, 4 )
+// reads the tile shape from the run descriptor.  NT: threads; 128 unless the
+// tile's blocks leave more warps resident in larger CTAs (pk_config).
+template < int PUSH, int MOVE, bool DETECT, typename JT, int TN, int NT >
+__global__ void __launch_bounds__( NT, pk_ctas( NT ) )
 k_particles( const Item * __restrict__ items, const SpDev * __restrict__ sps,
              const RunDev * __restrict__ runs, const int * __restrict__ shifts )
 {
@@ -362,16 +577,17 @@ k_particles( const Item * __restrict__ items, const SpDev * __restrict__ sps,
     const int t = it.tile;
     const int nchunk = S.nchunk;
 
-    // shared memory: [E tile][B tile][tile current (JT; fixed point: hi
-    //                words then lo words)][mbarrier][energy partials][crossing queues]
+    // shared memory: [E tile][B tile][tile current (JT; fixed point: words, then wrap counts)]
+    //                [crossing queues][factors][energy partials][mbarrier]
     constexpr bool FIX = std::is_same<JT, int>::value;
     constexpr int JW = FIX ? 2 : 1;
     float * sE = reinterpret_cast<float *>( smem_raw );
     float * sB = sE + 3 * tv;
     JT * sJ = reinterpret_cast<JT *>( sB + 3 * tv );
-    uint64_t * bar = reinterpret_cast<uint64_t *>( sJ + 3 * tv * JW );
-    double * sred = reinterpret_cast<double *>( bar + 1 );
-    CrossQueue * xq = reinterpret_cast<CrossQueue *>( sred + PK_THREADS / 32 );
+    CrossQueue * xq = reinterpret_cast<CrossQueue *>( sJ + 3 * tv * JW );
+    PairFactors & fac = *reinterpret_cast<PairFactors *>( xq + NT / 32 );
+    double * sred = reinterpret_cast<double *>( &fac + 1 );
+    uint64_t * bar = reinterpret_cast<uint64_t *>( sred + NT / 32 );
 
     const int np = S.np[ t ];
     const int off = S.off[ t ];
@@ -391,22 +607,46 @@ k_particles( const Item * __restrict__ items, const SpDev * __restrict__ sps,
     __shared__ int s_dir[9];
     if ( DETECT && threadIdx.x < 9 ) s_dir[ threadIdx.x ] = 0;
 
-    if ( PUSH ) {
-        if ( threadIdx.x == 0 ) {
-            mbar_init( bar, 1 );
-            fence_mbar_init();
-        }
-        __syncthreads();
-        if ( threadIdx.x == 0 ) {
-            const uint32_t bytes = 12u * tv;
-            mbar_arrive_expect_tx( bar, 2 * bytes );
-            bulk_g2s( sE, R.E + (size_t) t * 3 * tv, bytes, bar );
-            bulk_g2s( sB, R.B + (size_t) t * 3 * tv, bytes, bar );
-        }
+    // the factors, one by each of the second warp's first lanes (loaded before
+    // the copies are issued: a wait for them here would be on every CTA's way):
+    // half of q dx / dt and q / 2 (for q vz / 2) times the fixed-point scale
+    // (exact power-of-two products)
+    float factor = 0.0f;
+    if ( threadIdx.x >= 32 && threadIdx.x < 38 ) {
+        const int k = threadIdx.x - 32;
+        const float v = k == 0 ? S.dt_dx : k == 1 ? S.dt_dy : k == 2 ? S.qnx : k == 3 ? S.qny : k == 4 ? S.alpha : S.q;
+        factor = k == 2 || k == 3 || k == 5 ? 0.5f * v * ( FIX ? S.jscale : 1.0f ) : v;
     }
+    if ( PUSH && threadIdx.x == 0 ) {
+        mbar_init( bar, 1 );
+        fence_mbar_init();
+        const uint32_t bytes = 12u * tv;
+        mbar_arrive_expect_tx( bar, 2 * bytes );
+        bulk_g2s( sE, R.E + (size_t) t * 3 * tv, bytes, bar );
+        bulk_g2s( sB, R.B + (size_t) t * 3 * tv, bytes, bar );
+    }
+    constexpr bool NEED_U = PUSH || MOVE;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    CrossQueue & Q = xq[ warp ];
+    // the tile's particles: six arrays `stride` bytes apart
+    char * const pa = reinterpret_cast<char *>( S.A.cell + off );
+    const size_t stride = S.A.stride;
+    // the lines of the warp's 64 particles from `at` on into L1: lanes 0-17
+    // touch the first, the 33rd and the last of them in each array
+    const int pfe = lane % 3 == 0 ? 0 : lane % 3 == 1 ? 32 : WP - 1;
+    const char * const pf = pa + ( lane < 18 ? lane / 3 : 0 ) * stride + 4 * pfe;
+    auto prefetch = [&]( int at ) {
+        if ( lane < 18 && at + pfe < end ) asm volatile( "prefetch.global.L1 [%0];" :: "l"( pf + 4 * (size_t) at ) );
+    };
+    prefetch( begin + warp * WP );
+    if ( threadIdx.x >= 32 && threadIdx.x < 38 ) ( &fac.dt_dx )[ threadIdx.x - 32 ] = both( factor );
+    if ( threadIdx.x == 38 ) fac.nz = both( -0.0f );
     if ( MOVE == 2 ) {
-        for ( int i = threadIdx.x; i < 3 * tv * JW; i += blockDim.x ) sJ[i] = (JT) 0;
+        float4 * z = reinterpret_cast<float4 *>( sJ );          // 3 tv words are a multiple of 16 bytes
+        constexpr int W = 3 * JW * sizeof( JT ) / 4;
+        for ( int i = threadIdx.x; i < W * tv / 4; i += NT ) z[i] = make_float4( 0.f, 0.f, 0.f, 0.f );
     }
+    __syncthreads();
     if ( PUSH ) {
         // an expired wait: the item's particles, current and energy are left
         // as they were (the step is reported failed)
@@ -414,8 +654,6 @@ k_particles( const Item * __restrict__ items, const SpDev * __restrict__ sps,
             if ( threadIdx.x == 0 ) S.energy[ eidx ] = 0.0;
             return;
         }
-    } else {
-        __syncthreads();
     }
 
     const int ys = TN ? TN + 3 : R.extx;
@@ -426,7 +664,6 @@ k_particles( const Item * __restrict__ items, const SpDev * __restrict__ sps,
     const int nxx = TN ? TN : R.nxx, nxy = TN ? TN : R.nxy;
     const int tx = t % R.ntx, ty = t / R.ntx;
     const int shift = ( MOVE && shifts ) ? shifts[ it.sp ] : 0;
-    const bool euler = ( PUSH == 2 );
 
     // reflecting walls handled here (species.cpp:1854-1989): lower rule on the
     // first tile column, upper rule on the last one; x first, then y.
@@ -436,184 +673,229 @@ k_particles( const Item * __restrict__ items, const SpDev * __restrict__ sps,
     const int ryu = ( MOVE && ty != 0 && ty == R.nty - 1 && ( S.bc[2] > 1 || S.bc[3] > 1 ) && S.bc[3] == 2 );
     const bool walls = ( rxl | rxu | ryl | ryu ) != 0;
 
-    const float alpha = S.alpha;
-    // current factors: half of q dx / dt, and q / 2 (for q vz / 2), times the
-    // fixed-point scale (exact power-of-two products)
-    const float jsf = FIX ? S.jscale : 1.0f;
-    const float dt_dx = S.dt_dx, dt_dy = S.dt_dy, qhalf = 0.5f * S.q * jsf;
-    const float qnxx = 0.5f * S.qnx * jsf, qnxy = 0.5f * S.qny * jsf;
+    // the pair quotient alpha / gamma is exact for these (time step and mass
+    // over charge of any plasma)
+    const bool alpha_ok = fabsf( S.alpha ) > 1e-18f && fabsf( S.alpha ) < 1e18f;
     const JAcc ja = { S.jscale, 3 * tv };
 
-    uint32_t * __restrict__ pc = S.A.cell + off;
-    float * __restrict__ pxx = S.A.xx + off;
-    float * __restrict__ pxy = S.A.xy + off;
-    float * __restrict__ pux = S.A.ux + off;
-    float * __restrict__ puy = S.A.uy + off;
-    float * __restrict__ puz = S.A.uz + off;
-
     double energy = 0.0;
-    const int lane = threadIdx.x & 31;
-    const unsigned lt_mask = ( 1u << lane ) - 1u;
-    CrossQueue & Q = xq[ threadIdx.x >> 5 ];
-    int qh = 0, qt = 0;                         // warp-uniform ring head / tail
+    int qh = 0, qn = 0;                         // warp-uniform ring head and fill
 
-    // Groups of FLUSH_PARTICLES: with the fixed-point tile current the
-    // accumulators are flushed between groups (at most 3 additions per
-    // particle and entry, well below the 2^16 the words can take).
-    for ( int g0 = begin; g0 < end; g0 += FLUSH_PARTICLES ) {
-        if constexpr ( FIX && MOVE == 2 ) {
-            if ( g0 != begin ) jfix_flush( reinterpret_cast<int *>( sJ ), 3 * tv, R.Jdep + (size_t) t * 3 * tv, S.jscale_inv );
+    for ( int w0 = begin + warp * WP; w0 < end; w0 += PK_PPT * NT ) {
+        const int i0 = w0 + lane;
+        uint32_t c[PK_PPT]; float x0[PK_PPT], x1[PK_PPT], u0[PK_PPT], u1[PK_PPT], u2[PK_PPT];
+        int leave_dir[PK_PPT];
+#pragma unroll
+        for ( int k = 0; k < PK_PPT; k++ ) {
+            c[k] = 0; x0[k] = x1[k] = u0[k] = u1[k] = u2[k] = 0.f;
+            if ( i0 + 32 * k < end ) {
+                const char * src = pa + 4 * (size_t) ( i0 + 32 * k );
+                c[k] = *reinterpret_cast<const uint32_t *>( src );
+                x0[k] = *reinterpret_cast<const float *>( src + stride );
+                x1[k] = *reinterpret_cast<const float *>( src + 2 * stride );
+                if ( NEED_U ) {
+                    u0[k] = *reinterpret_cast<const float *>( src + 3 * stride );
+                    u1[k] = *reinterpret_cast<const float *>( src + 4 * stride );
+                    u2[k] = *reinterpret_cast<const float *>( src + 5 * stride );
+                }
+            }
         }
-        const int gend = min( end, g0 + FLUSH_PARTICLES );
-        for ( int b0 = g0; b0 < gend; b0 += PK_PPT * PK_THREADS ) {
-            uint32_t c[PK_PPT] = {}; float x0[PK_PPT], x1[PK_PPT], u0[PK_PPT], u1[PK_PPT], u2[PK_PPT];
-            int leave_dir[PK_PPT];
+        // Sorted particles sit inside their tile; anything else (only
+        // reachable by moving twice without a sort) is flagged and left
+        // untouched so no field or current access leaves the tile block.
+        // TN x TN tiles (TN a power of two): both 16-bit cell coordinates
+        // inside [0, TN) exactly when no bit above TN - 1 is set.  Lanes
+        // without a particle compute on cell 0 of the tile and store nothing.
+        bool valid[PK_PPT];
+        int ix[PK_PPT], iy[PK_PPT];
+        {
+            bool bad = false;
 #pragma unroll
             for ( int k = 0; k < PK_PPT; k++ ) {
-                const int i = b0 + k * PK_THREADS + threadIdx.x;
-                if ( i < end ) {
-                    c[k] = pc[i]; x0[k] = pxx[i]; x1[k] = pxy[i];
-                    if ( PUSH || MOVE ) { u0[k] = pux[i]; u1[k] = puy[i]; u2[k] = puz[i]; }
-                }
-            }
-#pragma unroll
-            for ( int k = 0; k < PK_PPT; k++ ) {
-                const int i = b0 + k * PK_THREADS + threadIdx.x;
-                bool valid = i < end;
-                bool cross = false;
-                leave_dir[k] = 4;
-                int ix = 0, iy = 0, oix = 0, oiy = 0;
-                float d0 = 0.f, d1 = 0.f, qz = 0.f, ox = 0.f, oy = 0.f;
+                valid[k] = i0 + 32 * k < end;
+                ix[k] = cell_x( c[k] ); iy[k] = cell_y( c[k] );
                 if ( PUSH || MOVE ) {
-                    ix = cell_x( c[k] ); iy = cell_y( c[k] );
-                    // Sorted particles sit inside their tile; anything else (only
-                    // reachable by moving twice without a sort) is flagged and left
-                    // untouched so no field or current access leaves the tile block.
-                    // TN x TN tiles (TN a power of two): both 16-bit cell
-                    // coordinates inside [0, TN) exactly when no bit above TN - 1 is set
-                    const bool bad = valid && ( ( TN > 0 && ( TN & ( TN - 1 ) ) == 0 )
+                    const bool out = ( TN > 0 && ( TN & ( TN - 1 ) ) == 0 )
                                    ? ( c[k] & ~( (uint32_t) ( TN - 1 ) * 0x10001u ) ) != 0
-                                   : ( ix < 0 || ix >= nxx || iy < 0 || iy >= nxy ) );
-                    const unsigned mbad = __ballot_sync( 0xffffffffu, bad );
-                    if ( mbad ) {
-                        if ( lane == __ffs( mbad ) - 1 ) atomicOr( R.status, ST_BAD_CELL );
-                        valid = valid && !bad;
-                    }
-                } else if ( valid ) {
-                    ix = cell_x( c[k] ); iy = cell_y( c[k] );
-                }
-                if ( valid ) {
-                    if ( PUSH ) {
-                        float ex, ey, ez, bx, by, bz;
-                        interpolate_fld( Ec, Bc, ys, ix, iy, x0[k], x1[k], ex, ey, ez, bx, by, bz );
-                        if ( euler ) dudt_boris_euler( alpha, ex, ey, ez, bx, by, bz, u0[k], u1[k], u2[k], energy );
-                        else         dudt_boris( alpha, ex, ey, ez, bx, by, bz, u0[k], u1[k], u2[k], energy );
-                    }
-                    if ( MOVE ) {
-                        // species.cpp:1431-1489
-                        const float rg = rgamma( u0[k], u1[k], u2[k] );
-                        d0 = dt_dx * rg * u0[k];
-                        d1 = dt_dy * rg * u1[k];
-                        const float x1x = x0[k] + d0, x1y = x1[k] + d1;
-                        const int dix = ( ( x1x >= 0.5f ) - ( x1x < -0.5f ) );
-                        const int diy = ( ( x1y >= 0.5f ) - ( x1y < -0.5f ) );
-                        if ( MOVE == 2 ) {
-                            qz = qhalf * u2[k] * rg;
-                            cross = ( dix | diy ) != 0;
-                            if ( !cross )
-                                dep_current_seg( ix, iy, x0[k], x1[k], x1x, x1y, qnxx, qnxy, qz, Jc, ys, ja );
-                        }
-                        ox = x0[k]; oy = x1[k]; oix = ix; oiy = iy;
-                        x0[k] = x1x - dix; x1[k] = x1y - diy;
-                        ix += dix + shift; iy += diy;
-                        if ( walls ) {
-                            if ( rxl && ix < 0 )    { ix += 1; x0[k] = -x0[k]; u0[k] = -u0[k]; }
-                            if ( rxu && ix >= nxx ) { ix -= 1; x0[k] = -x0[k]; u0[k] = -u0[k]; }
-                            if ( ryl && iy < 0 )    { iy += 1; x1[k] = -x1[k]; u1[k] = -u1[k]; }
-                            if ( ryu && iy >= nxy ) { iy -= 1; x1[k] = -x1[k]; u1[k] = -u1[k]; }
-                        }
-                        c[k] = pack_cell( ix, iy );
-                    }
-                    if ( DETECT ) {
-                        const int xcross = ( ix >= nxx ) - ( ix < 0 );
-                        const int ycross = ( iy >= nxy ) - ( iy < 0 );
-                        leave_dir[k] = ( ycross + 1 ) * 3 + ( xcross + 1 );
-                    }
-                }
-                if ( MOVE == 2 ) {
-                    // queue cell-crossing particles (warp-uniform point)
-                    const unsigned m = __ballot_sync( 0xffffffffu, cross );
-                    if ( m ) {
-                        if ( cross ) {
-                            const int e = ( qt + __popc( m & lt_mask ) ) & ( XQ - 1 );
-                            Q.cell[e] = pack_cell( oix, oiy );
-                            Q.x0x[e] = ox; Q.x0y[e] = oy;
-                            Q.dx[e] = d0; Q.dy[e] = d1; Q.qvz[e] = qz;
-                        }
-                        qt += __popc( m );
-                        if ( qt - qh >= 32 ) {
-                            __syncwarp();
-                            drain_entry( Q, ( qh + lane ) & ( XQ - 1 ), qnxx, qnxy, Jc, ys, ja );
-                            qh += 32;
-                            __syncwarp();
-                        }
-                    }
+                                   : ( ix[k] < 0 || ix[k] >= nxx || iy[k] < 0 || iy[k] >= nxy );
+                    if ( out ) { bad = true; valid[k] = false; ix[k] = 0; iy[k] = 0; }
                 }
             }
+            if ( PUSH || MOVE ) {
+                const unsigned mbad = __ballot_sync( 0xffffffffu, bad );
+                if ( mbad && lane == __ffs( mbad ) - 1 ) atomicOr( R.status, ST_BAD_CELL );
+            }
+        }
+        if ( PUSH ) {
+            F2 ex, ey, ez, bx, by, bz;
+            const F2 al = lds2( fac.alpha ), nz = lds2( fac.nz );
+            interpolate_fld2( Ec, Bc, ys, ix[0], iy[0], ix[1], iy[1], x0[0], x1[0], x0[1], x1[1], nz, ex, ey, ez, bx, by, bz );
+            if constexpr ( PUSH == 2 ) {
+                float e[6][2];
+                unpack2( ex, e[0][0], e[0][1] ); unpack2( ey, e[1][0], e[1][1] ); unpack2( ez, e[2][0], e[2][1] );
+                unpack2( bx, e[3][0], e[3][1] ); unpack2( by, e[4][0], e[4][1] ); unpack2( bz, e[5][0], e[5][1] );
+#pragma unroll
+                for ( int k = 0; k < PK_PPT; k++ )
+                    if ( valid[k] ) dudt_boris_euler( lds1( fac.alpha ), e[0][k], e[1][k], e[2][k], e[3][k], e[4][k], e[5][k],
+                                                      u0[k], u1[k], u2[k], energy );
+            } else {
+                F2 vx = pack2( u0[0], u0[1] ), vy = pack2( u1[0], u1[1] ), vz = pack2( u2[0], u2[1] ), en;
+                if ( dudt_boris2( al, nz, ex, ey, ez, bx, by, bz, vx, vy, vz, en ) && alpha_ok ) {
+                    float e0, e1;
+                    unpack2( vx, u0[0], u0[1] ); unpack2( vy, u1[0], u1[1] ); unpack2( vz, u2[0], u2[1] );
+                    unpack2( en, e0, e1 );
+                    if ( valid[0] ) energy += (double) e0;
+                    if ( valid[1] ) energy += (double) e1;
+                } else {
+#pragma unroll
+                    for ( int k = 0; k < PK_PPT; k++ )
+                        if ( valid[k] ) {
+                            const float4 v = push_one( Ec, Bc, ys, ix[k], iy[k], x0[k], x1[k], lds1( fac.alpha ), u0[k], u1[k], u2[k] );
+                            u0[k] = v.x; u1[k] = v.y; u2[k] = v.z;
+                            energy += (double) v.w;
+                        }
+                }
+            }
+        }
+        prefetch( w0 + PK_PPT * NT );
+        // results go back as soon as they are known: values held to the end
+        // of the iteration would not fit the registers
+        char * const dst = pa + 4 * (size_t) i0;
+        auto put = [&]( int array, auto v0, auto v1 ) {
+            if ( valid[0] ) *reinterpret_cast<decltype( v0 ) *>( dst + array * stride ) = v0;
+            if ( valid[1] ) *reinterpret_cast<decltype( v0 ) *>( dst + array * stride + 128 ) = v1;
+        };
+        if ( PUSH ) { put( 3, u0[0], u0[1] ); put( 4, u1[0], u1[1] ); put( 5, u2[0], u2[1] ); }
+#pragma unroll
+        for ( int k = 0; k < PK_PPT; k++ ) leave_dir[k] = 4;
+        if ( MOVE ) {
+            // species.cpp:1431-1489
+            F2 rg;
+            const F2 ux2 = pack2( u0[0], u0[1] ), uy2 = pack2( u1[0], u1[1] ), uz2 = pack2( u2[0], u2[1] );
+            if ( !rgamma2( ux2, uy2, uz2, rg ) ) rg = pack2( rgamma( u0[0], u1[0], u2[0] ), rgamma( u0[1], u1[1], u2[1] ) );
+            F2 fx, fy;
+            lds2x2( fac.dt_dx, fx, fy );
+            const F2 nz = lds2( fac.nz );
+            const F2 dx2 = mul2( fx * rg, ux2, nz ), dy2 = mul2( fy * rg, uy2, nz );
+            const F2 xo = pack2( x0[0], x0[1] ), yo = pack2( x1[0], x1[1] );
+            const F2 xn = xo + dx2, yn = yo + dy2;
+            float n0[PK_PPT], n1[PK_PPT];
+            int dix[PK_PPT], diy[PK_PPT];
+            unpack2( xn, n0[0], n0[1] ); unpack2( yn, n1[0], n1[1] );
+            bool cross[PK_PPT];
+            float f0[PK_PPT], f1[PK_PPT];
+            int jx[PK_PPT], jy[PK_PPT];
 #pragma unroll
             for ( int k = 0; k < PK_PPT; k++ ) {
-                const int i = b0 + k * PK_THREADS + threadIdx.x;
-                if ( i < end ) {
-                    if ( MOVE ) { pc[i] = c[k]; pxx[i] = x0[k]; pxy[i] = x1[k]; }
-                    if ( PUSH || rxl || rxu ) pux[i] = u0[k];
-                    if ( PUSH || ryl || ryu ) puy[i] = u1[k];
-                    if ( PUSH ) puz[i] = u2[k];
+                dix[k] = ( ( n0[k] >= 0.5f ) - ( n0[k] < -0.5f ) );
+                diy[k] = ( ( n1[k] >= 0.5f ) - ( n1[k] < -0.5f ) );
+                cross[k] = valid[k] && ( dix[k] | diy[k] ) != 0;
+                jx[k] = ix[k]; jy[k] = iy[k];
+                f0[k] = n0[k] - dix[k]; f1[k] = n1[k] - diy[k];
+                ix[k] += dix[k] + shift; iy[k] += diy[k];
+                if ( walls ) {
+                    if ( rxl && ix[k] < 0 )    { ix[k] += 1; f0[k] = -f0[k]; u0[k] = -u0[k]; }
+                    if ( rxu && ix[k] >= nxx ) { ix[k] -= 1; f0[k] = -f0[k]; u0[k] = -u0[k]; }
+                    if ( ryl && iy[k] < 0 )    { iy[k] += 1; f1[k] = -f1[k]; u1[k] = -u1[k]; }
+                    if ( ryu && iy[k] >= nxy ) { iy[k] -= 1; f1[k] = -f1[k]; u1[k] = -u1[k]; }
                 }
             }
-
-            if ( DETECT ) {
-                // warp-aggregated append of leaver indices (one global atomic per warp)
-                int nl = 0;
+            const F2 qz2 = lds2( fac.qhalf ) * uz2 * rg;
+            if ( walls ) { put( 3, u0[0], u0[1] ); put( 4, u1[0], u1[1] ); }
+            put( 0, pack_cell( ix[0], iy[0] ), pack_cell( ix[1], iy[1] ) );
+            put( 1, f0[0], f0[1] );
+            put( 2, f1[0], f1[1] );
+            if ( MOVE == 2 ) {
+                float d0[PK_PPT], d1[PK_PPT], qz[PK_PPT];
+                unpack2( dx2, d0[0], d0[1] ); unpack2( dy2, d1[0], d1[1] ); unpack2( qz2, qz[0], qz[1] );
+                // queue cell-crossing particles (warp-uniform point)
 #pragma unroll
-                for ( int k = 0; k < PK_PPT; k++ ) nl += ( leave_dir[k] != 4 );
-                const unsigned any = __ballot_sync( 0xffffffffu, nl > 0 );
-                if ( any ) {
-                    int incl = nl;
-#pragma unroll
-                    for ( int o = 1; o < 32; o <<= 1 ) {
-                        const int v = __shfl_up_sync( 0xffffffffu, incl, o );
-                        if ( lane >= o ) incl += v;
+                for ( int k = 0; k < PK_PPT; k++ ) {
+                    const unsigned m = __ballot_sync( 0xffffffffu, cross[k] );
+                    if ( cross[k] ) {
+                        int e = qh + qn + __popc( m & ( ( 1u << lane ) - 1u ) );
+                        if ( e >= XQ ) e -= XQ;
+                        Q.cell[e] = pack_cell( jx[k], jy[k] );
+                        Q.x0x[e] = x0[k]; Q.x0y[e] = x1[k];
+                        Q.dx[e] = d0[k]; Q.dy[e] = d1[k]; Q.qvz[e] = qz[k];
                     }
-                    const int total = __shfl_sync( 0xffffffffu, incl, 31 );
-                    int wbase = 0;
-                    if ( lane == 31 ) wbase = atomicAdd( S.nidx + t, total );
-                    wbase = __shfl_sync( 0xffffffffu, wbase, 31 );
-                    int pos = wbase + incl - nl;
+                    qn += __popc( m );
+                }
+                if constexpr ( FIX ) {
+                    F2 hx, hy;
+                    lds2x2( fac.qnxx, hx, hy );
+                    dep_current_seg2( valid[0] && !cross[0], jx[0], jy[0], valid[1] && !cross[1], jx[1], jy[1],
+                                      xo, yo, xn, yn, hx, hy, qz2, Jc, ys, ja );
+                } else {
 #pragma unroll
-                    for ( int k = 0; k < PK_PPT; k++ ) {
-                        if ( leave_dir[k] != 4 ) {
-                            const int li = b0 + k * PK_THREADS + threadIdx.x;
-                            S.idx[ off + pos ] = li;
-                            // leaver outbox in buffer B (unused outside a repack),
-                            // so that the sort reads the leavers coalesced
-                            const size_t o = (size_t) off + pos;
-                            S.B.cell[o] = c[k]; S.B.xx[o] = x0[k]; S.B.xy[o] = x1[k];
-                            if ( PUSH || MOVE ) { S.B.ux[o] = u0[k]; S.B.uy[o] = u1[k]; S.B.uz[o] = u2[k]; }
-                            else { S.B.ux[o] = pux[li]; S.B.uy[o] = puy[li]; S.B.uz[o] = puz[li]; }
-                            pos++;
-                            // counted per direction when the target tile exists
-                            const int ttx = wrap_tile( tx + leave_dir[k] % 3 - 1, R.ntx, S.perx );
-                            const int tty = wrap_tile( ty + leave_dir[k] / 3 - 1, R.nty, S.pery );
-                            if ( ttx >= 0 && tty >= 0 ) atomicAdd( &s_dir[ leave_dir[k] ], 1 );
-                        }
+                    for ( int k = 0; k < PK_PPT; k++ )
+                        if ( valid[k] && !cross[k] )
+                            dep_current_seg( jx[k], jy[k], x0[k], x1[k], n0[k], n1[k], lds1( fac.qnxx ), lds1( fac.qnxy ),
+                                             qz[k], Jc, ys, ja );
+                }
+            }
+        }
+        if ( DETECT ) {
+#pragma unroll
+            for ( int k = 0; k < PK_PPT; k++ )
+                if ( valid[k] ) {
+                    const int xcross = ( ix[k] >= nxx ) - ( ix[k] < 0 );
+                    const int ycross = ( iy[k] >= nxy ) - ( iy[k] < 0 );
+                    leave_dir[k] = ( ycross + 1 ) * 3 + ( xcross + 1 );
+                }
+        }
+        if ( DETECT ) {
+            // warp-aggregated append of leaver indices (one global atomic per warp)
+            int nl = 0;
+#pragma unroll
+            for ( int k = 0; k < PK_PPT; k++ ) nl += ( leave_dir[k] != 4 );
+            const unsigned any = __ballot_sync( 0xffffffffu, nl > 0 );
+            if ( any ) {
+                int incl = nl;
+#pragma unroll
+                for ( int o = 1; o < 32; o <<= 1 ) {
+                    const int v = __shfl_up_sync( 0xffffffffu, incl, o );
+                    if ( lane >= o ) incl += v;
+                }
+                const int total = __shfl_sync( 0xffffffffu, incl, 31 );
+                int wbase = 0;
+                if ( lane == 31 ) wbase = atomicAdd( S.nidx + t, total );
+                wbase = __shfl_sync( 0xffffffffu, wbase, 31 );
+                int pos = wbase + incl - nl;
+#pragma unroll
+                for ( int k = 0; k < PK_PPT; k++ ) {
+                    if ( leave_dir[k] != 4 ) {
+                        const int li = i0 + 32 * k;
+                        S.idx[ off + pos ] = li;
+                        // leaver outbox in buffer B (unused outside a repack),
+                        // so that the sort reads the leavers coalesced
+                        const size_t o = (size_t) off + pos;
+                        // (this thread's own stores above)
+                        copy_particle( S.B, o, S.A, (size_t) off + li );
+                        pos++;
+                        // counted per direction when the target tile exists
+                        const int ttx = wrap_tile( tx + leave_dir[k] % 3 - 1, R.ntx, S.perx );
+                        const int tty = wrap_tile( ty + leave_dir[k] / 3 - 1, R.nty, S.pery );
+                        if ( ttx >= 0 && tty >= 0 ) atomicAdd( &s_dir[ leave_dir[k] ], 1 );
                     }
                 }
+            }
+        }
+        // full warps of queued crossings are split and deposited here, where
+        // the fewest values are live across the call
+        if ( MOVE == 2 ) {
+            while ( qn >= 32 ) {
+                __syncwarp();
+                drain_entry( Q, qh + lane < XQ ? qh + lane : qh + lane - XQ, lds1( fac.qnxx ), lds1( fac.qnxy ), Jc, ys, ja );
+                qh += 32; qn -= 32;
+                if ( qh >= XQ ) qh -= XQ;
+                __syncwarp();
             }
         }
     }
-    if ( MOVE == 2 && qt != qh ) {
+    if ( MOVE == 2 && qn > 0 ) {
         __syncwarp();
-        if ( lane < qt - qh ) drain_entry( Q, ( qh + lane ) & ( XQ - 1 ), qnxx, qnxy, Jc, ys, ja );
+        if ( lane < qn ) drain_entry( Q, qh + lane < XQ ? qh + lane : qh + lane - XQ, lds1( fac.qnxx ), lds1( fac.qnxy ), Jc, ys, ja );
     }
 
     if ( PUSH ) {
@@ -628,8 +910,7 @@ k_particles( const Item * __restrict__ items, const SpDev * __restrict__ sps,
         // round the FP64 or fixed-point tile current once per cell, into the E tile's place
         for ( int i = threadIdx.x; i < 3 * tv; i += blockDim.x ) {
             if constexpr ( FIX )
-                sE[i] = (float) jfix_value( sJ[i], reinterpret_cast<const unsigned int *>( sJ )[ 3 * tv + i ],
-                                            S.jscale_inv );
+                sE[i] = (float) jfix_value( sJ[i], sJ[ 3 * tv + i ], S.jscale_inv );
             else sE[i] = (float) sJ[i];
         }
         sJout = sE;
@@ -851,11 +1132,6 @@ __device__ __noinline__ void sort_plan( int sp, const SpDev & S, const RunDev & 
         S.nmove[1] += 1;
         rlist[ 1 + atomicAdd( rlist, 1 ) ] = sp;
     }
-}
-
-__device__ __forceinline__ void copy_particle( const PartArrays & d, size_t di, const PartArrays & s, size_t si ) {
-    d.cell[di] = s.cell[si]; d.xx[di] = s.xx[si]; d.xy[di] = s.xy[si];
-    d.ux[di] = s.ux[si]; d.uy[di] = s.uy[si]; d.uz[di] = s.uz[si];
 }
 
 constexpr int SORT_THREADS = 256;
@@ -1712,52 +1988,78 @@ k_reorder( const Item * __restrict__ items, const SpDev * __restrict__ sps, cons
 // ---------------------------------------------------------------------------
 namespace zb {
 
+// Threads per CTA of the particle kernel and CTAs per SM.  128 threads, which
+// waste less on few particles (4.2 M particles in 4,096 tiles 129 instead of 146
+// us), or 256 where a CTA gets more than PK_HEAVY particles (the tail of a
+// launch is as long as its fullest tile takes: a filamented sweep of 16 runs
+// 1357 against 1133 us), or what leaves more warps resident where the tile's
+// blocks are large (32x32 cells: 12, 16 and 24 warps of 128, 256 and 384).
+constexpr double PK_HEAVY = 4096.0;
+struct PkConfig { int threads, per_sm; size_t smem; };
+static size_t pk_smem( int tile_vol, int jacc, int threads ) {
+    return (size_t) ( jacc ? 12 : 9 ) * tile_vol * sizeof( float ) + sizeof( PairFactors ) +
+           ( threads / 32 ) * ( sizeof( CrossQueue ) + sizeof( double ) ) + 8;
+}
+static PkConfig pk_config( int tile_vol, int jacc, double per_cta ) {
+    PkConfig best{};
+    const int least = per_cta > PK_HEAVY ? 256 : 128;
+    for ( int threads = 128; threads <= 384; threads += 128 ) {
+        PkConfig c;
+        c.threads = threads;
+        c.smem = pk_smem( tile_vol, jacc, threads );
+        // 1 KB and the static shared memory per CTA are the system's and the kernel's own
+        c.per_sm = std::min( pk_ctas( threads ), (int) ( 227 * 1024 / ( c.smem + 1024 + 64 ) ) );
+        if ( threads == 128 || ( threads == least && c.per_sm > 0 ) || c.per_sm * c.threads > best.per_sm * best.threads ) best = c;
+    }
+    return best;
+}
+int particle_ctas_per_sm( int tile_vol, int jacc ) { return std::max( 1, pk_config( tile_vol, jacc, 0.0 ).per_sm ); }
+
+// Shared memory by which a tile's size is limited (at least what any launch
+// with 128 threads needs)
 size_t particle_smem_bytes( int tile_vol, int jacc ) {
-    return (size_t) ( jacc ? 12 : 9 ) * tile_vol * sizeof( float ) + 8 + ( PK_THREADS / 32 ) * sizeof( double ) +
-           ( PK_THREADS / 32 ) * sizeof( CrossQueue );
+    return (size_t) ( jacc ? 12 : 9 ) * tile_vol * sizeof( float ) + 8 + 8 * ( sizeof( double ) + 1536 );
 }
 
 typedef void ( *pk_fn )( const Item *, const SpDev *, const RunDev *, const int * );
 
-static pk_fn pick_particle_kernel( int push, int move, int detect, int jacc, int tile_n ) {
-    if ( tile_n == 16 && move == 2 && detect && ( push == 1 || push == 2 ) ) {
-        if ( jacc == 0 ) return push == 1 ? k_particles< 1, 2, true, float, 16 > : k_particles< 2, 2, true, float, 16 >;
-        if ( jacc == 1 ) return push == 1 ? k_particles< 1, 2, true, double, 16 > : k_particles< 2, 2, true, double, 16 >;
-        return push == 1 ? k_particles< 1, 2, true, int, 16 >
-                         : k_particles< 2, 2, true, int, 16 >;
+static pk_fn pick_particle_kernel( int push, int move, int detect, int jacc, int tile_n, int & threads ) {
+    if ( jacc == 2 && move == 2 && detect && tile_n == 16 && push && threads == 128 )
+        return push == 1 ? k_particles< 1, 2, true, int, 16, 128 > : k_particles< 2, 2, true, int, 16, 128 >;
+    if ( jacc == 2 && move == 2 && detect && tile_n == 16 && push && threads == 256 )
+        return push == 1 ? k_particles< 1, 2, true, int, 16, 256 > : k_particles< 2, 2, true, int, 16, 256 >;
+    if ( jacc == 2 && move == 2 && detect && push && threads == 256 )
+        return push == 1 ? k_particles< 1, 2, true, int, 0, 256 > : k_particles< 2, 2, true, int, 0, 256 >;
+    if ( jacc == 2 && move == 2 && detect && push && threads == 384 )
+        return push == 1 ? k_particles< 1, 2, true, int, 0, 384 > : k_particles< 2, 2, true, int, 0, 384 >;
+    threads = 128;
+    if ( jacc < 2 && move == 2 && detect && tile_n == 16 && push ) {
+        if ( jacc == 0 ) return push == 1 ? k_particles< 1, 2, true, float, 16, 128 > : k_particles< 2, 2, true, float, 16, 128 >;
+        return push == 1 ? k_particles< 1, 2, true, double, 16, 128 > : k_particles< 2, 2, true, double, 16, 128 >;
     }
-    if ( jacc == 1 && move == 2 ) {
-#define PKD( P, M, D ) if ( push == P && move == M && detect == D ) return k_particles< P, M, D, double >;
-        PKD( 1, 2, true ) PKD( 2, 2, true ) PKD( 0, 2, true )
-#undef PKD
-        return nullptr;
-    }
-    if ( jacc == 2 && move == 2 ) {
-#define PKX( P, M, D ) if ( push == P && move == M && detect == D ) return k_particles< P, M, D, int >;
-        PKX( 1, 2, true ) PKX( 2, 2, true ) PKX( 0, 2, true )
-#undef PKX
-        return nullptr;
-    }
-#define PK( P, M, D ) if ( push == P && move == M && detect == D ) return k_particles< P, M, D >;
-    PK( 1, 2, true ) PK( 2, 2, true )
-    PK( 1, 0, false ) PK( 2, 0, false )
-    PK( 0, 2, true ) PK( 0, 1, true ) PK( 0, 0, true )
-    PK( 1, 1, true ) PK( 2, 1, true )
+#define PK( P, M, D, T ) if ( push == P && move == M && detect == D ) return k_particles< P, M, D, T, 0, 128 >;
+    if ( jacc == 2 && move == 2 ) { PK( 1, 2, true, int ) PK( 2, 2, true, int ) PK( 0, 2, true, int ) return nullptr; }
+    if ( jacc == 1 && move == 2 ) { PK( 1, 2, true, double ) PK( 2, 2, true, double ) PK( 0, 2, true, double ) return nullptr; }
+    PK( 1, 2, true, float ) PK( 2, 2, true, float ) PK( 0, 2, true, float )
+    PK( 1, 0, false, float ) PK( 2, 0, false, float )
+    PK( 0, 1, true, float ) PK( 0, 0, true, float )
+    PK( 1, 1, true, float ) PK( 2, 1, true, float )
 #undef PK
     return nullptr;
 }
 
 cudaError_t launch_particles( cudaStream_t st, int push, int move, int detect, const Item * items, int nitems,
                               const SpDev * sps, const RunDev * runs, const int * shifts, int max_tile_vol,
-                              int jacc, int tile_n ) {
+                              int jacc, int tile_n, double per_cta ) {
     if ( move != 2 ) jacc = 0;
-    pk_fn f = pick_particle_kernel( push, move, detect, jacc, tile_n );
+    int threads = pk_config( max_tile_vol, jacc, per_cta ).threads;
+    pk_fn f = pick_particle_kernel( push, move, detect, jacc, tile_n, threads );
     if ( !f ) return cudaErrorInvalidValue;
-    const size_t smem = particle_smem_bytes( max_tile_vol, jacc );
+    const size_t smem = pk_smem( max_tile_vol, jacc, threads );
     if ( smem > 48 * 1024 )
         cudaFuncSetAttribute( (const void *) f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem );
     if ( nitems <= 0 ) return cudaSuccess;
-    f<<< nitems, PK_THREADS, smem, st >>>( items, sps, runs, shifts );
+    f<<< nitems, threads, smem, st >>>( items, sps, runs, shifts );
     return cudaGetLastError();
 }
 

@@ -49,6 +49,7 @@ struct PartArrays {
     uint32_t * cell;
     float * xx; float * xy;
     float * ux; float * uy; float * uz;
+    size_t stride;                // bytes from one array to the next (one allocation, in the order above)
 };
 
 // Per-species state.
