@@ -28,11 +28,12 @@ def _particles(geom, u_range, seed):
     return npt, ix, x, u.astype(np.float32)
 
 
-# 16x16 tiles (128 threads), generic ones in CTAs of 128, 256 and 384 threads (9x7, 35x21 and 32x32 cells)
-GEOMS = [((5, 5), (16, 16)), ((7, 3), (9, 7)), ((3, 7), (35, 21)), ((7, 3), (32, 32))]
+# square tiles of 8, 16 and 32 cells (their own instances, 32 in CTAs of 384 threads), generic ones in CTAs of 128
+# and 256 threads (9x7 and 35x21 cells)
+GEOMS = [((5, 5), (16, 16)), ((7, 3), (9, 7)), ((3, 7), (35, 21)), ((7, 3), (32, 32)), ((7, 6), (8, 8))]
 
 
-@pytest.mark.parametrize('tiles', GEOMS, ids=['16x16', '9x7', '35x21', '32x32'])
+@pytest.mark.parametrize('tiles', GEOMS, ids=['16x16', '9x7', '35x21', '32x32', '8x8'])
 @pytest.mark.parametrize('m_q,u_range,b', [(-1.0, (1e-3, 1e2), 2.0), (1.0, (1e-42, 1e-3), 1e-20), (-1.0, (1e2, 1e18), 1e3),
                                            (-1.0, (1e-3, 1e2), 1e17), (1e21, (1e-2, 1e1), 1.0), (-1e-19, (1e-2, 1e1), 1e-3)])
 def test_push_bit_exact(tiles, m_q, u_range, b):
@@ -52,7 +53,7 @@ def test_push_bit_exact(tiles, m_q, u_range, b):
     assert np.array_equal(o[3], g[3], equal_nan=True)
 
 
-@pytest.mark.parametrize('tiles', GEOMS, ids=['16x16', '9x7', '35x21', '32x32'])
+@pytest.mark.parametrize('tiles', GEOMS, ids=['16x16', '9x7', '35x21', '32x32', '8x8'])
 @pytest.mark.parametrize('u_range', [(1e-3, 1e-1), (0.5, 50.0)])
 def test_move_and_current(tiles, u_range):
     """Slow particles (few crossings) and fast ones (most particles cross, often two edges: the crossing queue

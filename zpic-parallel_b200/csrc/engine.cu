@@ -474,7 +474,7 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
             P.reorder_every = P.reorder_every > 0 ? std::min( P.reorder_every, every ) : every;
         // one accumulation mode per plan: the runs' own when they agree
         P.jacc = ( P.jacc < 0 || P.jacc == s->jacc ) ? s->jacc : 2;
-        const int tn = ( s->nxx == 16 && s->nxy == 16 ) ? 16 : 0;
+        const int tn = s->nxx == s->nxy && ( s->nxx == 8 || s->nxx == 16 || s->nxx == 32 ) ? s->nxx : 0;
         P.tile_n = ( P.tile_n < 0 || P.tile_n == tn ) ? tn : 0;
         for ( int t = 0; t < s->ntx * s->nty; t++ ) tiles.push_back( { (int) r, t } );
         for ( int k = 0; k < 4; k++ )
