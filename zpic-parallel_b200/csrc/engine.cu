@@ -122,9 +122,10 @@ enum Phase { PH_PARTICLES = 0, PH_SORT, PH_CURRENT, PH_FIELDS, PH_OTHER, PH_N };
 // Steps between in-tile reorders of the particles (option "reorder").  By
 // default (-1, automatic) every 50 steps, but never in a moving-window run:
 // there the plasma is cold and new particles arrive in injection order every
-// step, so the order hardly decays.  On the uniform plasma the particle
-// kernel takes 4.56 ms per step right after a reorder and 4.95 ms a hundred
-// steps later; a reorder costs ~3.9 ms, 0.08 ms per step at this interval.
+// step, so the order hardly decays.  On the uniform plasma (1024^2) the
+// particle kernel takes 1.08 ms per step right after a reorder, 1.16 and 1.18
+// ms 50 and 100 steps later; a reorder costs ~1 ms, 0.02 ms per step at this
+// interval.  Every 16 or 24 steps: no gain.
 constexpr int REORDER_DEFAULT = -1;
 constexpr int REORDER_AUTO_STEPS = 50;
 
@@ -803,8 +804,9 @@ static int maybe_reorder( Plan & P, cudaStream_t st, uint64_t * launches ) {
 static int plan_advance( Plan & P, cudaStream_t st, int nsteps, bool use_graph, uint64_t * launches ) {
     for ( auto * s : P.sims ) TRY( ensure_jdep_clean( s, st ) );
     // a step is captured when several are asked for at once, or when single
-    // steps keep coming: capturing costs about 0.5 ms, a replay saves about
-    // 10 us of launches
+    // steps keep coming: capturing costs about 0.2 ms, a replay saves 7 to 10 us
+    // of launches (64^2 and 210x132 cells: 47 -> 42, 74 -> 66 us per step), so
+    // by then the launches have cost as much as the capture would have
     if ( nsteps == 1 && P.single_steps < SINGLE_STEPS ) P.single_steps++;
     const bool can_graph = use_graph && ( nsteps > 1 || P.graph || P.single_steps >= SINGLE_STEPS );
     zpic_sim * ts = prof_sim( P );

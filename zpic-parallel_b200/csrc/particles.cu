@@ -2027,7 +2027,7 @@ typedef void ( *pk_fn )( const Item *, const SpDev *, const RunDev *, const int 
 
 static pk_fn pick_particle_kernel( int push, int move, int detect, int jacc, int tile_n, int & threads ) {
     // square tiles of 8, 16 and 32 cells, the sizes to choose from: 32x32 cells
-    // (512^2, 33.5 M particles) 771 -> 745 us per step
+    // (512^2, 33.5 M particles) 771 -> 748 us per step
     if ( jacc == 2 && move == 2 && detect && push ) {
 #define PK( N, T ) if ( tile_n == N && threads == T ) return push == 1 ? k_particles< 1, 2, true, int, N, T > : k_particles< 2, 2, true, int, N, T >;
         PK( 8, 128 ) PK( 16, 128 ) PK( 16, 256 ) PK( 32, 384 )
