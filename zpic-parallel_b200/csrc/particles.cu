@@ -650,9 +650,7 @@ k_particles( const Item * __restrict__ items, const SpDev * __restrict__ sps,
     if ( PUSH ) {
         // an expired wait: the item's particles, current and energy are left
         // as they were (the step is reported failed)
-        // (one poll of the limit stands for the issue of the copies, which cannot
-        // have arrived then; by now they often have)
-        if ( bulk_wait_or_abandon( bar, R.status, R.wait_limit - 1 ) ) {
+        if ( bulk_wait_or_abandon( bar, R.status, R.wait_limit ) ) {
             if ( threadIdx.x == 0 ) S.energy[ eidx ] = 0.0;
             return;
         }
