@@ -46,11 +46,14 @@ def test_push_bit_exact(tiles, m_q, u_range, b):
         s.set_grid('B', random_fields(s, 4, b))
         s.set_particles(0, *_particles(geom, u_range, 7))
         s.species_push(0)
-        sims.append(s.particles(0))
+        sims.append(s.particles(0) + (s.species_energy(0),))
     o, g = sims
     assert np.array_equal(o[0], g[0])
     # no tolerance: every operation is correctly rounded in both
     assert np.array_equal(o[3], g[3], equal_nan=True)
+    # the same non-negative terms, each one FP32 value, summed in FP64 in another order
+    if np.isfinite(o[4]):
+        assert abs(g[4] - o[4]) <= 2 * (int(o[0].sum()) + 8) * 2.0 ** -53 * abs(o[4])
 
 
 @pytest.mark.parametrize('tiles', GEOMS, ids=['16x16', '9x7', '35x21', '32x32', '8x8'])

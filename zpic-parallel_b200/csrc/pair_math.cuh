@@ -33,10 +33,14 @@ __device__ __forceinline__ F2 neg2( F2 a ) { float x, y; unpack2( a, x, y ); ret
 // step on the exact remainder that fma gives (P. Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
 // Dev. 34, 1990).  The same floats as the IEEE operations, without their tests
-// of the argument's range at each call: every float of [1, 2^96) was compared
-// for the root and the reciprocal, every one of [1, 2^12) with 64 numerators
-// for the quotient; the theorem behind the last step holds for all numerators
-// whose quotient and remainder are normal numbers.
+// of the argument's range at each call: tests/test_device_functions_gpu.py
+// compares every float of [1, 2^96) for the root and the reciprocal, and for the
+// quotient every significand of the divisor with 64 numerators each.  The
+// theorem behind the last step asks for a quotient and a remainder that are
+// normal numbers.  The kernel's two quotients are alpha / gamma, with |alpha| in
+// (1e-18, 1e18), and the energy term utsq / (gamma + 1): where utsq is too small
+// for that, gamma is 1 and the divisor exactly 2, and the same test compares that
+// term for every float utsq of [0, 2^96).
 constexpr float QLIM = 7.9e28f;             // about 2^96
 __device__ __forceinline__ F2 sqrt2( F2 x ) {
     float a, b, ra, rb;
