@@ -2,6 +2,7 @@
 copy changes its path (direct, one lane, several lanes, ragged last parts), from several threads at once;
 single-step calls give the same run before and after they switch to a captured step."""
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -16,10 +17,11 @@ def _sim(ntiles, nx):
     return zb.Simulation(ntiles, nx, (ntiles[0] * nx[0] * dx, ntiles[1] * nx[1] * dx), 0.05)
 
 
-# bytes of one grid: 364 * 12 = 4,368 per 16x16 tile; 64 KiB lies between 15 and 16 tiles, 512 KiB (a chunk)
-# between 120 and 121, 1 MiB at 240.05, 2 MiB at 480.1, 4 MiB at 960.2
-@pytest.mark.parametrize('ntiles', [(1, 1), (5, 3), (4, 4), (12, 10), (11, 11), (16, 15), (241, 1), (30, 16), (37, 13),
-                                    (31, 31), (64, 61)])
+# bytes of one grid: 364 * 12 = 4,368 per 16x16 tile; 64 KiB lies between 15 and 16 tiles, 224 KiB (a chunk)
+# between 52 and 53, 448 KiB between 105 and 106, 2 MiB and 12 MiB (all lanes) between 480 and 481, 2,880 and 2,881
+@pytest.mark.parametrize('ntiles', [(1, 1), (5, 3), (4, 4), (52, 1), (53, 1), (15, 7), (53, 2), (12, 10),
+                                    (11, 11), (16, 15), (241, 1), (30, 16), (37, 13), (32, 30), (31, 31), (64, 45), (43, 67),
+                                    (64, 61)])
 def test_grid_round_trip(ntiles):
     s = _sim(ntiles, (16, 16))
     a = np.random.default_rng(ntiles[0]).random((ntiles[0] * ntiles[1], s.tile_vol, 3), np.float32)
@@ -70,6 +72,29 @@ def test_threads_share_the_lanes():
     s = _sim((30, 20), (16, 16))
     s.set_grid('E', data[0])
     assert np.array_equal(s.grid('E'), data[0])
+
+
+def _median_ms(f, n):
+    v = []
+    for _ in range(n):
+        t = time.perf_counter()
+        keep = f()
+        v.append((time.perf_counter() - t) * 1e3)
+        del keep
+    return sorted(v)[n // 2]
+
+
+def test_first_read_out_of_a_simulation_costs_no_more_than_the_next():
+    """Simulations one after another, each read out and closed: what a read-out needs is made in microseconds.
+    (2.1 to 5.7 ms when it made four streams and 4 MB of pinned memory, against 0.04 ms for the second.)"""
+    first, second = [], []
+    for _ in range(9):
+        s = _sim((8, 8), (16, 16))
+        s.synchronize()
+        first.append(_median_ms(lambda: s.grid('E'), 1))
+        second.append(_median_ms(lambda: s.grid('E'), 1))
+        s.close()
+    assert sorted(first)[4] <= sorted(second)[4] + 0.5
 
 
 def test_single_steps_equal_a_run():

@@ -1,11 +1,12 @@
 // readback.cu -- device-to-host copies of diagnostics.
 //
-// A driver copy into pageable memory goes through one staging thread: 8 GB/s
-// into fresh memory, of the link's 55.  Here a copy is cut into up to LANES
-// parts, each with its own stream, two pinned chunks and host thread, so
-// that the copies over the link, the page faults of the destination and the
-// host-side copies overlap: 35.8 MB (one field of 2048x1024 cells) into fresh
-// memory takes 2.5 ms instead of 7.9.
+// A driver copy into pageable memory goes through one staging thread: 16 GB/s
+// into pages that the process has just used, 2 to 8 into pages that it has to
+// fault in, of the link's 55.  So a copy goes through two pinned chunks here, and
+// a large one is cut into LANES parts, each with its own stream, chunks and host
+// thread, so that the copies over the link, the page faults of the destination
+// and the host-side copies overlap: 35.8 MB (one field of 2048x1024 cells) into
+// fresh memory takes 2.5 ms instead of 7.9, 1.1 MB 0.43 instead of 0.55.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -21,49 +22,55 @@ namespace zb {
 namespace {
 
 constexpr int LANES = 4;
-constexpr size_t CHUNK = 512 * 1024;          // pinned bytes per slot (two slots per lane)
+constexpr size_t CHUNK = 224 * 1024;          // pinned bytes per slot (two slots per lane: all lanes within 2 MB)
 constexpr size_t SMALL = 64 * 1024;           // the driver's own path is as good below
 constexpr size_t PER_LANE = 1024 * 1024;      // a further lane (host thread) pays from this many bytes on
 
 struct Lane {
-    cudaStream_t st = nullptr;
+    cudaStream_t st = nullptr;                // none for the first lane: it copies on the caller's stream
     cudaEvent_t done[2] = { nullptr, nullptr };
     char * buf = nullptr;                     // two chunks
 };
 
-// The lanes of one device: 4 MB of pinned memory, made at the first copy that
-// uses them and given back when the device's last simulation is destroyed.
+// The lanes of one device, made when they are first used and given back when the
+// device's last simulation is destroyed.  The first read-out of a simulation
+// pays for them, so they are made to cost little: the first lane needs no stream,
+// and the driver cuts pinned buffers from blocks of 2 MB, 1.3 ms each, of which
+// every simulation holds one for its scratch: the lanes' 1.75 MB fit the rest of
+// it (4 MB of buffers and four streams made at once took 2.1 to 5 ms, and 0.9 ms
+// when they were given back; now 0.01 ms, and 0.2 for the three streams of a wide copy).
 struct Pool {
     std::mutex busy;
     Lane lane[LANES];
     cudaEvent_t ready = nullptr;
-    bool made = false;
+    int made = 0;
     int users = 0;
 
-    cudaError_t make() {
-        if ( made ) return cudaSuccess;
-        cudaError_t e = cudaEventCreateWithFlags( &ready, cudaEventDisableTiming );
-        for ( auto & l : lane ) {
-            if ( e == cudaSuccess ) e = cudaStreamCreateWithFlags( &l.st, cudaStreamNonBlocking );
+    // lanes [0, n) are there, or as many as could be made
+    void make( int n ) {
+        cudaError_t e = cudaSuccess;
+        if ( !ready && n > 1 ) e = cudaEventCreateWithFlags( &ready, cudaEventDisableTiming );
+        while ( made < n && e == cudaSuccess ) {
+            Lane & l = lane[made];
+            if ( made > 0 ) e = cudaStreamCreateWithFlags( &l.st, cudaStreamNonBlocking );
             for ( int k = 0; k < 2; k++ )
                 if ( e == cudaSuccess ) e = cudaEventCreateWithFlags( &l.done[k], cudaEventDisableTiming );
             if ( e == cudaSuccess ) e = cudaHostAlloc( (void **) &l.buf, 2 * CHUNK, cudaHostAllocPortable );
+            if ( e == cudaSuccess ) made++; else free_lane( l );
         }
-        made = true;
-        if ( e != cudaSuccess ) drop();
-        return e;
+        if ( e != cudaSuccess ) cudaGetLastError();
+    }
+    void free_lane( Lane & l ) {
+        if ( l.st ) { cudaStreamSynchronize( l.st ); cudaStreamDestroy( l.st ); }
+        for ( int k = 0; k < 2; k++ ) if ( l.done[k] ) cudaEventDestroy( l.done[k] );
+        if ( l.buf ) cudaFreeHost( l.buf );
+        l = Lane{};
     }
     void drop() {
-        if ( !made ) return;
-        for ( auto & l : lane ) {
-            if ( l.st ) { cudaStreamSynchronize( l.st ); cudaStreamDestroy( l.st ); }
-            for ( int k = 0; k < 2; k++ ) if ( l.done[k] ) cudaEventDestroy( l.done[k] );
-            if ( l.buf ) cudaFreeHost( l.buf );
-            l = Lane{};
-        }
+        for ( auto & l : lane ) free_lane( l );
         if ( ready ) cudaEventDestroy( ready );
         ready = nullptr;
-        made = false;
+        made = 0;
     }
 };
 
@@ -71,7 +78,7 @@ std::mutex g_pools_mutex;
 std::map<int, std::unique_ptr<Pool>> g_pools;
 
 // One lane's part: chunk k comes over the link while chunk k - 1 is copied out.
-cudaError_t run_lane( int device, Lane & l, char * dst, const char * src, size_t bytes ) {
+cudaError_t run_lane( int device, Lane & l, cudaStream_t st, char * dst, const char * src, size_t bytes ) {
     cudaError_t e = cudaSetDevice( device );
     if ( e != cudaSuccess ) return e;
     const size_t n = ( bytes + CHUNK - 1 ) / CHUNK;
@@ -79,8 +86,8 @@ cudaError_t run_lane( int device, Lane & l, char * dst, const char * src, size_t
         const int b = (int) ( k & 1 );
         if ( k < n ) {
             const size_t at = k * CHUNK, len = std::min( CHUNK, bytes - at );
-            e = cudaMemcpyAsync( l.buf + b * CHUNK, src + at, len, cudaMemcpyDeviceToHost, l.st );
-            if ( e == cudaSuccess ) e = cudaEventRecord( l.done[b], l.st );
+            e = cudaMemcpyAsync( l.buf + b * CHUNK, src + at, len, cudaMemcpyDeviceToHost, st );
+            if ( e == cudaSuccess ) e = cudaEventRecord( l.done[b], st );
             if ( e != cudaSuccess ) break;
         }
         if ( k > 0 ) {
@@ -90,7 +97,7 @@ cudaError_t run_lane( int device, Lane & l, char * dst, const char * src, size_t
             std::memcpy( dst + at, l.buf + ( 1 - b ) * CHUNK, len );
         }
     }
-    if ( e != cudaSuccess ) cudaStreamSynchronize( l.st );     // nothing of this copy is left in flight
+    if ( e != cudaSuccess ) cudaStreamSynchronize( st );       // nothing of this copy is left in flight
     return e;
 }
 
@@ -133,17 +140,21 @@ cudaError_t copy_to_host( int device, cudaStream_t st, void * dst, const void * 
     }
     if ( !pool ) return copy_plain( st, dst, src, bytes );
     std::unique_lock<std::mutex> own( pool->busy, std::try_to_lock );
-    if ( !own.owns_lock() || pool->make() != cudaSuccess ) { cudaGetLastError(); return copy_plain( st, dst, src, bytes ); }
-    const unsigned cores = std::thread::hardware_concurrency();
-    const int lanes = (int) std::max<size_t>( 1, std::min<size_t>( { (size_t) LANES, bytes / PER_LANE, (size_t) std::max( 1u, cores ) } ) );
-    cudaError_t e = cudaEventRecord( pool->ready, st );
-    for ( int k = 0; k < lanes && e == cudaSuccess; k++ ) e = cudaStreamWaitEvent( pool->lane[k].st, pool->ready, 0 );
+    if ( !own.owns_lock() ) return copy_plain( st, dst, src, bytes );
+    const size_t cores = std::max( 1u, std::thread::hardware_concurrency() );
+    const int want = (int) std::max<size_t>( 1, std::min<size_t>( { (size_t) LANES, bytes / PER_LANE, cores } ) );
+    pool->make( want );
+    if ( pool->made == 0 ) return copy_plain( st, dst, src, bytes );
+    const int lanes = std::min( want, pool->made );
+    cudaError_t e = cudaSuccess;
+    if ( lanes > 1 ) e = cudaEventRecord( pool->ready, st );
+    for ( int k = 1; k < lanes && e == cudaSuccess; k++ ) e = cudaStreamWaitEvent( pool->lane[k].st, pool->ready, 0 );
     if ( e != cudaSuccess ) return e;
     const size_t part = ( ( bytes + lanes - 1 ) / lanes + 4095 ) & ~(size_t) 4095;
     cudaError_t err[LANES];
     auto work = [&]( int k ) {
         const size_t at = std::min( bytes, k * part ), len = std::min( part, bytes - at );
-        err[k] = len ? run_lane( device, pool->lane[k], (char *) dst + at, (const char *) src + at, len ) : cudaSuccess;
+        err[k] = len ? run_lane( device, pool->lane[k], k ? pool->lane[k].st : st, (char *) dst + at, (const char *) src + at, len ) : cudaSuccess;
     };
     std::thread th[LANES];
     int started = 1;
