@@ -478,8 +478,11 @@ constexpr int WP = 64;                      // particles of one warp iteration (
 constexpr int PK_PPT = 2;
 // CTAs per SM that the registers allow, at 80 a thread.  (7 of 128 threads at
 // 72 spill: 128x128 Weibel set-up 57 -> 56 us per step, but 4096x512 wakefield
-// 534 -> 543 and 24x14-cell tiles 34 -> 36.)
-constexpr int pk_ctas( int threads ) { return 768 / threads; }
+// 534 -> 543 and 24x14-cell tiles 34 -> 36.)  At 72 for the Boris push of 16x16
+// tiles with FP32 or FP64 tile currents, whose additions (compare-and-swap loops)
+// are bound by their latency: 512^2 cells, 16.8 M particles 588 -> 546 and 731 -> 693
+// us per step (24x14-cell tiles 125 -> 131, exact rotation 118 -> 122: not there).
+constexpr int pk_ctas( int threads, bool cas16 ) { return ( cas16 ? 896 : 768 ) / threads; }
 
 // The species' factors, each in both halves of a pair; read from shared memory
 // where they are used rather than held in registers through the loop.
@@ -509,7 +512,7 @@ __device__ __forceinline__ float lds1( const F2 & p ) {
 // reads the tile shape from the run descriptor.  NT: threads; 128 unless the
 // tile's blocks leave more warps resident in larger CTAs (pk_config).
 template < int PUSH, int MOVE, bool DETECT, typename JT, int TN, int NT >
-__global__ void __launch_bounds__( NT, pk_ctas( NT ) )
+__global__ void __launch_bounds__( NT, pk_ctas( NT, PUSH == 1 && MOVE == 2 && TN == 16 && !std::is_same<JT, int>::value ) )
 k_particles( const Item * __restrict__ items, const SpDev * __restrict__ sps,
              const RunDev * __restrict__ runs, const int * __restrict__ shifts )
 {
@@ -1937,8 +1940,13 @@ namespace zb {
 // waste less on few particles (4.2 M particles in 4,096 tiles 129 instead of 146
 // us), or 256 where a CTA gets more than PK_HEAVY particles (the tail of a
 // launch is as long as its fullest tile takes: a filamented sweep of 16 runs
-// 1357 against 1133 us), or what leaves more warps resident where the tile's
-// blocks are large (32x32 cells: 12, 16 and 24 warps of 128, 256 and 384).
+// 1357 against 1133 us; not with FP32 and FP64 tile currents, whose 128-thread
+// CTAs leave more warps: 67 M particles 2047 against 2187 and 2618 against 2783 us), or what leaves more warps resident where the tile's
+// blocks are large (32x32 cells: 12, 16 and 24 warps of 128, 256 and 384; 64x64
+// cells: 4, 6 and 7 warps of 128, 192 and 224).  Every instance has these sizes:
+// with 128 threads for the FP32 and FP64 tile currents 32x32-cell tiles took 312 and
+// 339 us per step instead of 204 and 211, 64x64 302 instead of 202 with the
+// fixed-point one.
 constexpr double PK_HEAVY = 4096.0;
 struct PkConfig { int threads, per_sm; size_t smem; };
 static size_t pk_smem( int tile_vol, int jacc, int threads ) {
@@ -1947,13 +1955,13 @@ static size_t pk_smem( int tile_vol, int jacc, int threads ) {
 }
 static PkConfig pk_config( int tile_vol, int jacc, double per_cta ) {
     PkConfig best{};
-    const int least = per_cta > PK_HEAVY ? 256 : 128;
-    for ( int threads = 128; threads <= 384; threads += 128 ) {
+    const int least = jacc == 2 && per_cta > PK_HEAVY ? 256 : 128;
+    for ( const int threads : { 128, 192, 224, 256, 384 } ) {
         PkConfig c;
         c.threads = threads;
         c.smem = pk_smem( tile_vol, jacc, threads );
-        // 1 KB and the static shared memory per CTA are the system's and the kernel's own
-        c.per_sm = std::min( pk_ctas( threads ), (int) ( 227 * 1024 / ( c.smem + 1024 + 64 ) ) );
+        // of an SM's 228 KB every CTA takes 1 KB for the system and the kernel's static shared memory
+        c.per_sm = std::min( pk_ctas( threads, false ), (int) ( 228 * 1024 / ( c.smem + 1024 + 64 ) ) );
         if ( threads == 128 || ( threads == least && c.per_sm > 0 ) || c.per_sm * c.threads > best.per_sm * best.threads ) best = c;
     }
     return best;
@@ -1968,30 +1976,32 @@ size_t particle_smem_bytes( int tile_vol, int jacc ) {
 
 typedef void ( *pk_fn )( const Item *, const SpDev *, const RunDev *, const int * );
 
-static pk_fn pick_particle_kernel( int push, int move, int detect, int jacc, int tile_n, int & threads ) {
-    // square tiles of 8, 16 and 32 cells, the sizes to choose from: 32x32 cells
-    // (512^2, 33.5 M particles) 771 -> 748 us per step
-    if ( jacc == 2 && move == 2 && detect && push ) {
-#define PK( N, T ) if ( tile_n == N && threads == T ) return push == 1 ? k_particles< 1, 2, true, int, N, T > : k_particles< 2, 2, true, int, N, T >;
-        PK( 8, 128 ) PK( 16, 128 ) PK( 16, 256 ) PK( 32, 384 )
+template < int PUSH, int MOVE, bool DETECT, typename JT, int TN > static pk_fn pk_threads( int threads ) {
+    switch ( threads ) {
+    case 128: return k_particles< PUSH, MOVE, DETECT, JT, TN, 128 >;
+    case 192: return k_particles< PUSH, MOVE, DETECT, JT, TN, 192 >;
+    case 224: return k_particles< PUSH, MOVE, DETECT, JT, TN, 224 >;
+    case 256: return k_particles< PUSH, MOVE, DETECT, JT, TN, 256 >;
+    case 384: return k_particles< PUSH, MOVE, DETECT, JT, TN, 384 >;
+    }
+    return nullptr;
+}
+
+static pk_fn pick_particle_kernel( int push, int move, int detect, int jacc, int tile_n, int threads ) {
+    if ( move == 2 && detect && push ) {
+        // square tiles of 8, 16 and 32 cells, the sizes to choose from: 32x32 cells
+        // (512^2, 33.5 M particles) 771 -> 748 us per step
+#define PK( J, N, T, NT ) if ( jacc == J && tile_n == N && threads == NT ) return push == 1 ? k_particles< 1, 2, true, T, N, NT > : k_particles< 2, 2, true, T, N, NT >;
+        PK( 2, 8, int, 128 ) PK( 2, 16, int, 128 ) PK( 2, 16, int, 256 ) PK( 2, 32, int, 384 )
+        PK( 0, 16, float, 128 ) PK( 0, 16, float, 256 ) PK( 1, 16, double, 128 ) PK( 1, 16, double, 256 )
 #undef PK
     }
-    if ( jacc == 2 && move == 2 && detect && push && threads == 256 )
-        return push == 1 ? k_particles< 1, 2, true, int, 0, 256 > : k_particles< 2, 2, true, int, 0, 256 >;
-    if ( jacc == 2 && move == 2 && detect && push && threads == 384 )
-        return push == 1 ? k_particles< 1, 2, true, int, 0, 384 > : k_particles< 2, 2, true, int, 0, 384 >;
-    threads = 128;
-    if ( jacc < 2 && move == 2 && detect && tile_n == 16 && push ) {
-        if ( jacc == 0 ) return push == 1 ? k_particles< 1, 2, true, float, 16, 128 > : k_particles< 2, 2, true, float, 16, 128 >;
-        return push == 1 ? k_particles< 1, 2, true, double, 16, 128 > : k_particles< 2, 2, true, double, 16, 128 >;
-    }
-#define PK( P, M, D, T ) if ( push == P && move == M && detect == D ) return k_particles< P, M, D, T, 0, 128 >;
+#define PK( P, M, D, T ) if ( push == P && move == M && detect == D ) return pk_threads< P, M, D, T, 0 >( threads );
     if ( jacc == 2 && move == 2 ) { PK( 1, 2, true, int ) PK( 2, 2, true, int ) PK( 0, 2, true, int ) return nullptr; }
     if ( jacc == 1 && move == 2 ) { PK( 1, 2, true, double ) PK( 2, 2, true, double ) PK( 0, 2, true, double ) return nullptr; }
     PK( 1, 2, true, float ) PK( 2, 2, true, float ) PK( 0, 2, true, float )
     PK( 1, 0, false, float ) PK( 2, 0, false, float )
     PK( 0, 1, true, float ) PK( 0, 0, true, float )
-    PK( 1, 1, true, float ) PK( 2, 1, true, float )
 #undef PK
     return nullptr;
 }
@@ -2000,7 +2010,7 @@ cudaError_t launch_particles( cudaStream_t st, int push, int move, int detect, c
                               const SpDev * sps, const RunDev * runs, const int * shifts, int max_tile_vol,
                               int jacc, int tile_n, double per_cta ) {
     if ( move != 2 ) jacc = 0;
-    int threads = pk_config( max_tile_vol, jacc, per_cta ).threads;
+    const int threads = pk_config( max_tile_vol, jacc, per_cta ).threads;
     pk_fn f = pick_particle_kernel( push, move, detect, jacc, tile_n, threads );
     if ( !f ) return cudaErrorInvalidValue;
     const size_t smem = pk_smem( max_tile_vol, jacc, threads );
