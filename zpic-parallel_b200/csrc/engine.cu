@@ -212,7 +212,7 @@ struct Plan {
     bool needs_bc_or_filter = false;
     bool sum_in_yee = true;         // the field solve sums the deposits (run_current_fields)
     bool filter_in_one = true;      // every run has a current filter that one kernel takes (run_current)
-    int single_steps = 0;           // steps asked for one at a time so far (up to SINGLE_STEPS)
+    int single_steps = 0;           // steps asked for one at a time since the plan was built (up to SINGLE_STEPS)
     cudaGraphExec_t graph = nullptr;
     int graph_kernels = 0;
     // in-graph phase timing (profile 2): the captured graph and its event-record
@@ -244,6 +244,7 @@ struct Plan {
         if ( side ) { cudaStreamDestroy( side ); side = nullptr; }
         for ( auto & g : mw_graphs ) cudaGraphExecDestroy( g.second.first );
         mw_graphs.clear();
+        single_steps = 0;           // the next graph has to pay for its capture again
         dfree( runs_d ); dfree( sps_d ); dfree( k1_items_d[0] ); dfree( k1_items_d[1] );
         dfree( sort_items_d ); dfree( segs_d ); dfree( rlist_d ); dfree( tile_items_d ); dfree( spk1_d );
         built = false;
