@@ -37,7 +37,7 @@ cudaError_t launch_unpack( cudaStream_t, int, int, int, const SpDev *, const int
                            const float * );
 cudaError_t launch_gather( cudaStream_t, int, int, const SpDev *, const RunDev *, const int *, int, float, float, int, float * );
 cudaError_t launch_dep_charge( cudaStream_t, int, int, const SpDev *, const RunDev *, float *, int, int );
-cudaError_t launch_phasespace( cudaStream_t, int, int, const SpDev *, const RunDev *, PhaSpec, float * );
+cudaError_t launch_phasespace( cudaStream_t, int, int, const SpDev *, const RunDev *, PhaSpec, double, float * );
 cudaError_t launch_energy_sum( cudaStream_t, const SpDev *, int, int, double * );
 cudaError_t launch_np_stats( cudaStream_t, const SpDev *, int, unsigned long long * );
 cudaError_t launch_reorder( cudaStream_t, const Item *, int, const SpDev *, const RunDev *, int );
@@ -2158,7 +2158,7 @@ int zpic_b200_species_phasespace( zpic_sim * s, int32_t sp, int32_t quant0, cons
     TRY( w.get( s, w.bytes_of<float>( nbins ) ) );
     float * d = w.take<float>( nbins );
     CK( cudaMemsetAsync( d, 0, nbins * sizeof( float ), s->stream ) );
-    CK( launch_phasespace( s->stream, sp, h->ntiles, s->plan.sps_d, s->plan.runs_d, p, d ) );
+    CK( launch_phasespace( s->stream, sp, h->ntiles, s->plan.sps_d, s->plan.runs_d, p, (double) h->np_bound, d ) );
     s->launches += 1;
     CK( copy_to_host( s->device, s->stream, out, d, nbins * sizeof( float ) ) );
     return check_status( s );

@@ -2106,26 +2106,38 @@ cudaError_t launch_dep_charge( cudaStream_t st, int sp, int ntiles, const SpDev 
     return cudaGetLastError();
 }
 
+// particles: about how many the species has
 cudaError_t launch_phasespace( cudaStream_t st, int sp, int ntiles, const SpDev * sps, const RunDev * runs,
-                              PhaSpec p, float * out ) {
+                              PhaSpec p, double particles, float * out ) {
     const int nbins = p.n0 * ( p.q1 >= 0 ? p.n1 : 1 );
     const size_t one = (size_t) nbins * sizeof( float );
+    int dev = 0, sms = 148;
+    cudaGetDevice( &dev );
+    cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
     // Private copies per CTA when the phase space fits in shared memory: up to
     // 24 KB of them, a copy per warp at most, in four CTAs of 512 threads per
     // SM; a larger phase space once in one CTA of 1024 threads (256x128 bins,
     // 2.4 M particles: 137 us with 256 threads, 256 bins 53 us with one copy).
     p.smem = one <= 200 * 1024;
     const bool large = one > 48 * 1024;
-    const int threads = !p.smem ? 256 : large ? 1024 : 512;
-    const int copies = !p.smem || large ? 1 : (int) std::max<size_t>( 1, std::min<size_t>( threads / 32, 24 * 1024 / one ) );
+    int threads = !p.smem ? 256 : large ? 1024 : 512, per_sm = large && p.smem ? 1 : 4;
+    // In between, where 16 warps would share a copy, smaller CTAs with a copy each
+    // if the particles outnumber the bins of all of them: tiles put their
+    // particles into few bins of x, and warps at the same bin wait for one another
+    // (64x64 bins of x and uz, 21 M particles: 1,730 us with 512 threads, 1,545
+    // with 256, 1,050 with 128; 128x96 1,038, 777 and 716, but of ux and uy 324, 301
+    // and 471).
+    if ( !large && one > 12 * 1024 ) {
+        const int t = one > 26 * 1024 ? 256 : 128;
+        const int n = std::min( 2048 / t, (int) ( 226 * 1024 / ( one + 1024 ) ) );
+        if ( particles >= (double) n * sms * nbins ) { threads = t; per_sm = n; }
+    }
+    const int copies = !p.smem || large || threads < 512 ? 1 : (int) std::max<size_t>( 1, std::min<size_t>( threads / 32, 24 * 1024 / one ) );
     const size_t smem = p.smem ? one * copies : 0;
     if ( smem > 48 * 1024 )
         cudaFuncSetAttribute( (const void *) k_phasespace, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem );
-    int dev = 0, sms = 148;
-    cudaGetDevice( &dev );
-    cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
     // two work items per CTA at least
-    const int ctas = large && p.smem ? sms : 4 * sms;
+    const int ctas = per_sm * sms;
     const int parts = std::max( 1, std::min( 64, ( 2 * ctas + ntiles - 1 ) / ntiles ) );
     k_phasespace<<< std::min( ntiles * parts, ctas ), threads, smem, st >>>( sp, sps, runs, p, parts, copies, out );
     return cudaGetLastError();
