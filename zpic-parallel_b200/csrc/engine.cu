@@ -159,6 +159,7 @@ struct HSpecies {
     int ntiles = 0;
     uint32_t max_part = 0;
     uint64_t np_bound = 0;    // upper bound of the particle count (capacity checks)
+    int np_max = 0;           // particles of the fullest tile when they were last set
     int grows = 0;            // particle-buffer growths so far
     int pool_h = 0;           // host copy of the pool start at the last upload (copy source)
     SpDev d{};                // descriptor (device pointers)
@@ -200,7 +201,7 @@ struct Plan {
     Item * spk1_d = nullptr;
     std::vector<int> sp_k1_off, sp_k1_n, sp_sort_off, sp_sort_n, sp_seg_off, sp_seg_n;
     TileItem * tile_items_d = nullptr; int n_tiles = 0;
-    double per_cta = 0;             // particles per CTA of the particle kernel, in the fullest tiles of a full plasma
+    double per_cta = 0;             // particles per CTA of the particle kernel, in the fullest tiles
     int max_tile_vol = 0;
     int max_cells = 0, max_guard = 0;   // cells and guard cells of the largest tile
     int max_nxy = 0;                // tile rows (cells in y) of the tallest tile
@@ -286,6 +287,7 @@ struct zpic_sim {
     bool use_graph = true;
     int reorder_every = REORDER_DEFAULT;
     int chunks_opt = 0;
+    double chunk_particles = 0, chunk_fullest = 0;      // what CTAs per tile were chosen for (set_chunks)
     int jacc = 2;                   // fixed-point tile current (option "jacc")
     double pool_frac = 0.25;        // share of free particle capacity kept as the pool (option "pool_fraction")
     double reloc_room = 0.5;        // room for a relocated tile, share of its count (option "relocation_room")
@@ -373,37 +375,51 @@ struct Workspace {
     ~Workspace() { if ( own ) dfree( p ); }
 };
 
+// Particles that auto_chunks chooses by: of all tiles, and of the fullest one.  A
+// moving window's plasma is the one that will fill it.
+struct ChunkLoad { uint64_t tiles = 0; double particles = 0, fullest = 0; };
+static double full_tile( const zpic_sim * s, const HSpecies * h ) {
+    const double nominal = (double) h->ppc[0] * h->ppc[1] * s->nxx * s->nxy;
+    return s->emf_mw.active && h->dens.type != ZPIC_DENSITY_NONE ? std::max<double>( nominal, h->np_max ) : h->np_max;
+}
+static void add_load( ChunkLoad & l, const zpic_sim * s ) {
+    for ( auto * h : s->species ) {
+        const double full = full_tile( s, h );
+        l.tiles += h->ntiles;
+        l.particles += s->emf_mw.active ? full * h->ntiles : std::min<double>( h->np_bound, full * h->ntiles );
+        l.fullest = std::max( l.fullest, full );
+    }
+}
+
 // Chunks (CTAs) per tile for the particle kernel (the reference splits tiles
 // over blockIdx.z the same way, cuda/em2d/species.cpp:924-937), by the time a
-// launch would take: its waves of resident CTAs (per_sm of them on an SM),
-// each CTA with its fixed part (set-up, field staging, write-back of the tile
-// current) and its particles, plus the cost of every CTA launched.  Measured:
-// 15.6 ps per particle with all slots busy, 5 us fixed, 8.2 ns per CTA.  Small runs
-// get one full wave rather than two and a bit (128x128 Weibel set-up, 4 CTAs
-// per tile instead of 10: 41 against 47 us per step while it is uniform; 64x64
-// cells 33 -> 26 us), few large tiles several (512 tiles of 32x32 cells, 6
-// instead of 3: 861 -> 831 us).
-static int auto_chunks( uint64_t ntiles, double particles_per_tile, int per_sm, int opt ) {
+// launch would take: its waves of resident CTAs, each CTA with its fixed part
+// (set-up, field staging, write-back of the tile current) and its share of the
+// fullest tile's particles, plus the cost of every CTA launched. Measured: 15.6 ps
+// per particle with all slots busy, 5 us fixed, 8.2 ns per CTA.  Small runs get one
+// full wave rather than two and a bit (128x128 Weibel set-up, 6 CTAs per tile
+// instead of 10: 40 against 44 us per step while it is uniform).
+// By the particles there are, wherever they are: with CTAs for tiles filled as ppc
+// says, 64 per cell set on 4x4 and 8x8 tiles of a species of 1 per cell took 60 and
+// 87 us per step instead of 35 and 52, and a sphere in the middle of 32x32 tiles 87
+// instead of 64; a CTA that finds no particles costs 1.2 ns.
+static int auto_chunks( const ChunkLoad & l, int per_sm, int opt ) {
     if ( opt > 0 ) return opt;
     int dev = 0; cudaGetDevice( &dev );
     int sms = 148; cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
     // with enough tiles one CTA each, whose current does not depend on the order
     // of its sums: the same from run to run
-    if ( ntiles >= (uint64_t) sms * 8 ) return 1;
+    if ( l.tiles >= (uint64_t) sms * 8 ) return 1;
     const double slots = (double) sms * per_sm;
+    const double busy = l.fullest > 0 ? std::min<double>( l.tiles, l.particles / l.fullest ) : 0;
     int best = 1; double best_us = 0;
     for ( int c = 1; c <= 64; c++ ) {
-        const double ctas = (double) ntiles * c;
-        const double us = std::ceil( ctas / slots ) * ( 15.6e-6 * slots * particles_per_tile / c + 5.0 ) + 0.0082 * ctas;
+        const double ctas = busy * c;
+        const double us = std::ceil( ctas / slots ) * ( 15.6e-6 * slots * l.fullest / c + 5.0 ) + 0.0082 * ctas + 0.0012 * ( l.tiles * c - ctas );
         if ( c == 1 || us < best_us ) { best = c; best_us = us; }
     }
     return best;
 }
-
-// Particles per tile of a full plasma, and CTAs of the particle kernel per SM
-// (six of 128 threads by their registers; large tiles fewer by their shared memory).
-static double nominal_per_tile( const zpic_sim * s, const HSpecies * h ) { return (double) h->ppc[0] * h->ppc[1] * s->nxx * s->nxy; }
-static int ctas_per_sm( const zpic_sim * s ) { return particle_ctas_per_sm( s->run.tile_vol, s->jacc ); }
 
 // CTAs per tile of the particle kernel ("chunks" option): n > 0 for every
 // tile; 0, the automatic choice, for every tile; -1 balanced: a tile of
@@ -413,15 +429,37 @@ static int ctas_per_sm( const zpic_sim * s ) { return particle_ctas_per_sm( s->r
 // plasma fills the tiles (faster once a Weibel plasma has filamented, slower
 // for uniform plasmas and for runs with many empty tiles).
 static void set_chunks( zpic_sim * s ) {
-    int ntot = 0; uint64_t np = 0; double nominal = 0;
-    for ( auto * h : s->species ) { ntot += h->ntiles; np += h->np_bound; nominal += h->ntiles * nominal_per_tile( s, h ); }
-    const int base = auto_chunks( std::max( 1, ntot ), nominal / std::max( 1, ntot ), ctas_per_sm( s ), std::max( 0, s->chunks_opt ) );
+    int ntot = 0; uint64_t np = 0;
+    for ( auto * h : s->species ) { ntot += h->ntiles; np += h->np_bound; }
+    ChunkLoad load;
+    add_load( load, s );
+    s->chunk_particles = load.particles; s->chunk_fullest = load.fullest;
+    const int base = auto_chunks( load, particle_ctas_per_sm( s->run.tile_vol, s->jacc ), std::max( 0, s->chunks_opt ) );
     for ( auto * h : s->species ) {
         if ( s->chunks_opt >= 0 ) { h->d.nchunk = base; h->d.chunk_target = 0; continue; }
         h->d.nchunk = std::min( 64, 2 * base );
         const uint64_t per_tile = ( np + ntot - 1 ) / std::max( 1, ntot );
         h->d.chunk_target = (int) std::max<uint64_t>( 256, ( per_tile + base - 1 ) / base );
     }
+}
+
+// The same once particles have been set, where their number or that of the
+// fullest tile is half as much again or less than that for which it was chosen
+// (plans and graphs are built anew when the choice changes).
+static void rechoose_chunks( zpic_sim * s ) {
+    ChunkLoad now;
+    add_load( now, s );
+    auto near = []( double a, double b ) { return a <= 1.5 * b && b <= 1.5 * a; };
+    if ( near( now.particles, s->chunk_particles ) && near( now.fullest, s->chunk_fullest ) ) return;
+    bool other = false;
+    std::vector<std::pair<int, int>> was;
+    for ( auto * h : s->species ) was.push_back( { h->d.nchunk, h->d.chunk_target } );
+    set_chunks( s );
+    for ( size_t k = 0; k < was.size(); k++ )
+        other = other || was[k] != std::make_pair( s->species[k]->d.nchunk, s->species[k]->d.chunk_target );
+    if ( !other ) return;
+    s->plan.release();
+    s->layout_gen++;                // a batch chooses from all of its runs
 }
 
 static int upload_run( zpic_sim * s ) {
@@ -453,15 +491,6 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
     P.tile_n = -1;
     P.needs_bc_or_filter = false;
     P.sum_in_yee = true; P.filter_in_one = true;
-    uint64_t total_tiles = 0; double nominal = 0; int per_sm = 4;
-    for ( auto * s : sims ) {
-        per_sm = std::min( per_sm, ctas_per_sm( s ) );
-        for ( auto * sp : s->species ) { total_tiles += sp->ntiles; nominal += sp->ntiles * nominal_per_tile( s, sp ); }
-    }
-    // a batch chooses its CTAs per tile from all of its tiles; a single
-    // simulation keeps the choice made for it
-    const int batch_chunks = chunks_override > 0 ? chunks_override
-                           : sims.size() > 1 ? auto_chunks( std::max<uint64_t>( 1, total_tiles ), nominal / std::max<uint64_t>( 1, total_tiles ), per_sm, 0 ) : 0;
     for ( size_t r = 0; r < sims.size(); r++ ) {
         zpic_sim * s = sims[r];
         runs.push_back( s->run );
@@ -486,13 +515,22 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
         if ( !filter_smem_bytes( s->run.extx, s->run.exty, s->fdir, filter_npass( s ) ) ) P.filter_in_one = false;
         for ( int k = 0; k < 4; k++ ) if ( s->cur_bc[k] > ZPIC_CURRENT_BC_PERIODIC ) P.sum_in_yee = false;
     }
+    // a batch chooses its CTAs per tile from all of its tiles; a single
+    // simulation keeps the choice made for it
+    int batch_chunks = chunks_override;
+    if ( batch_chunks <= 0 && sims.size() > 1 ) {
+        ChunkLoad load;
+        int per_sm = 4;
+        for ( auto * s : sims ) { add_load( load, s ); per_sm = std::min( per_sm, particle_ctas_per_sm( s->run.tile_vol, s->jacc ) ); }
+        batch_chunks = auto_chunks( load, per_sm, 0 );
+    }
     for ( size_t r = 0; r < sims.size(); r++ ) {
         zpic_sim * s = sims[r];
         for ( size_t k = 0; k < s->species.size(); k++ ) {
             HSpecies * sp = s->species[k];
             SpDev d = sp->d;
-            if ( batch_chunks ) { d.nchunk = batch_chunks; d.chunk_target = 0; }
-            P.per_cta = std::max( P.per_cta, nominal_per_tile( s, sp ) / d.nchunk );
+            if ( batch_chunks > 0 ) { d.nchunk = batch_chunks; d.chunk_target = 0; }
+            P.per_cta = std::max( P.per_cta, full_tile( s, sp ) / d.nchunk );
             d.run = (int) r;
             const int gi = (int) P.sps_h.size();
             P.sps_h.push_back( d );
@@ -1020,6 +1058,7 @@ static int species_upload( zpic_sim * s, HSpecies * sp, const std::vector<int> &
     CK( cudaStreamSynchronize( st ) );
     dfree( one ); dfree( poff_d );
     sp->np_bound = total;
+    sp->np_max = *std::max_element( np.begin(), np.end() );
     sp->sort_pending = false;
     sp->counters_dirty = false;
     return ZPIC_OK;
@@ -1532,6 +1571,7 @@ int zpic_b200_sim_set_moving_window( zpic_sim * s ) {
             species_params( s, sp );
         }
     }
+    set_chunks( s );
     TRY( upload_run( s ) );
     return ZPIC_OK;
 }
@@ -1553,7 +1593,7 @@ int zpic_b200_sim_set_option( zpic_sim * s, const char * key, double v ) {
     else if ( k == "jacc" ) {
         const int j = (int) v;
         if ( j < 0 || j > 2 || j != v ) return fail( ZPIC_E_INVALID, "jacc must be 0, 1 or 2" );
-        if ( j != s->jacc ) { s->jacc = j; s->plan.release(); }
+        if ( j != s->jacc ) { s->jacc = j; set_chunks( s ); s->plan.release(); }
     }
     else if ( k == "reorder" ) {
         const int r = (int) v;
@@ -2070,6 +2110,7 @@ int zpic_b200_species_set( zpic_sim * s, int32_t sp, const int32_t * np, const i
     // a set larger than the buffer grows it (with a fifth to spare)
     if ( need + 4ull * h->ntiles > h->max_part ) TRY( species_grow( s, h, ( need + 4ull * h->ntiles ) * 6 / 5 ) );
     TRY( species_upload( s, h, n, ix, x, u ) );
+    rechoose_chunks( s );
     return ZPIC_OK;
 }
 
