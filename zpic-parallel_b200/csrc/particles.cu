@@ -1942,8 +1942,9 @@ namespace zb {
 // launch is as long as its fullest tile takes: a filamented sweep of 16 runs
 // 1357 against 1133 us; not with FP32 and FP64 tile currents, whose 128-thread
 // CTAs leave more warps: 67 M particles 2047 against 2187 and 2618 against 2783 us), or what leaves more warps resident where the tile's
-// blocks are large (32x32 cells: 12, 16 and 24 warps of 128, 256 and 384; 64x64
-// cells: 4, 6 and 7 warps of 128, 192 and 224).  Every instance has these sizes:
+// blocks are large (32x32 cells: 12, 16 and 24 warps of 128, 256 and 384), or 192 or
+// 224 where none of these fits but one CTA of 128 (64x64 cells: 6 and 7 warps; where
+// 256 threads leave as many, as for 24x24 cells, 192 took 4 % longer).  Every instance has these sizes:
 // with 128 threads for the FP32 and FP64 tile currents 32x32-cell tiles took 312 and
 // 339 us per step instead of 204 and 211, 64x64 302 instead of 202 with the
 // fixed-point one.
@@ -1956,7 +1957,8 @@ static size_t pk_smem( int tile_vol, int jacc, int threads ) {
 static PkConfig pk_config( int tile_vol, int jacc, double per_cta ) {
     PkConfig best{};
     const int least = jacc == 2 && per_cta > PK_HEAVY ? 256 : 128;
-    for ( const int threads : { 128, 192, 224, 256, 384 } ) {
+    for ( const int threads : { 128, 256, 384, 192, 224 } ) {
+        if ( threads % 128 && best.per_sm * best.threads >= 256 ) break;
         PkConfig c;
         c.threads = threads;
         c.smem = pk_smem( tile_vol, jacc, threads );
