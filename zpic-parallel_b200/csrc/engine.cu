@@ -395,27 +395,32 @@ static void add_load( ChunkLoad & l, const zpic_sim * s ) {
 // over blockIdx.z the same way, cuda/em2d/species.cpp:924-937), by the time a
 // launch would take: its waves of resident CTAs, each CTA with its fixed part
 // (set-up, field staging, write-back of the tile current) and its share of the
-// fullest tile's particles, plus the cost of every CTA launched. Measured: 15.6 ps
-// per particle with all slots busy, 5 us fixed, 8.2 ns per CTA.  Small runs get one
-// full wave rather than two and a bit (128x128 Weibel set-up, 6 CTAs per tile
-// instead of 10: 40 against 44 us per step while it is uniform).
+// fullest tile's particles, plus the cost of every CTA launched.  15.6 ps per
+// particle with all slots busy (of the smallest CTAs; a fifth more where shares of more
+// than PK_HEAVY particles get larger and fewer ones, whose tail is longer), 5 us fixed, 8.2
+// ns per CTA.  Particle kernel by CTAs per tile: 8x8 tiles of 1,024 particles
+// 22.6 us with 1, 13.8 with 5, 19.6 with 20; two species of 4,096 there 51.0 with 1,
+// 25.1 with 6, 32.9 with 20; 32x32 such tiles 124 with 1, 109 with 2, 125 with 6; 16x16
+// tiles of 16,384 123 with 1, 111 with 3, 108 with 6; 384 of them 155 with 1 and 2,
+// 150 with 4.
 // By the particles there are, wherever they are: with CTAs for tiles filled as ppc
 // says, 64 per cell set on 4x4 and 8x8 tiles of a species of 1 per cell took 60 and
 // 87 us per step instead of 35 and 52, and a sphere in the middle of 32x32 tiles 87
 // instead of 64; a CTA that finds no particles costs 1.2 ns.
-static int auto_chunks( const ChunkLoad & l, int per_sm, int opt ) {
+static int auto_chunks( const ChunkLoad & l, int tile_vol, int jacc, int opt ) {
     if ( opt > 0 ) return opt;
     int dev = 0; cudaGetDevice( &dev );
     int sms = 148; cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
     // with enough tiles one CTA each, whose current does not depend on the order
     // of its sums: the same from run to run
     if ( l.tiles >= (uint64_t) sms * 8 ) return 1;
-    const double slots = (double) sms * per_sm;
+    const double slots = (double) sms * particle_ctas_per_sm( tile_vol, jacc );
     const double busy = l.fullest > 0 ? std::min<double>( l.tiles, l.particles / l.fullest ) : 0;
     int best = 1; double best_us = 0;
     for ( int c = 1; c <= 64; c++ ) {
-        const double ctas = busy * c;
-        const double us = std::ceil( ctas / slots ) * ( 15.6e-6 * slots * l.fullest / c + 5.0 ) + 0.0082 * ctas + 0.0012 * ( l.tiles * c - ctas );
+        const double ctas = busy * c, share = l.fullest / c;
+        const double ps = jacc == 2 && share > PK_HEAVY ? 15.6e-6 * 1.2 : 15.6e-6;
+        const double us = std::ceil( ctas / slots ) * ( ps * slots * share + 5.0 ) + 0.0082 * ctas + 0.0012 * ( l.tiles * c - ctas );
         if ( c == 1 || us < best_us ) { best = c; best_us = us; }
     }
     return best;
@@ -434,7 +439,7 @@ static void set_chunks( zpic_sim * s ) {
     ChunkLoad load;
     add_load( load, s );
     s->chunk_particles = load.particles; s->chunk_fullest = load.fullest;
-    const int base = auto_chunks( load, particle_ctas_per_sm( s->run.tile_vol, s->jacc ), std::max( 0, s->chunks_opt ) );
+    const int base = auto_chunks( load, s->run.tile_vol, s->jacc, std::max( 0, s->chunks_opt ) );
     for ( auto * h : s->species ) {
         if ( s->chunks_opt >= 0 ) { h->d.nchunk = base; h->d.chunk_target = 0; continue; }
         h->d.nchunk = std::min( 64, 2 * base );
@@ -520,9 +525,8 @@ static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunk
     int batch_chunks = chunks_override;
     if ( batch_chunks <= 0 && sims.size() > 1 ) {
         ChunkLoad load;
-        int per_sm = 4;
-        for ( auto * s : sims ) { add_load( load, s ); per_sm = std::min( per_sm, particle_ctas_per_sm( s->run.tile_vol, s->jacc ) ); }
-        batch_chunks = auto_chunks( load, per_sm, 0 );
+        for ( auto * s : sims ) add_load( load, s );
+        batch_chunks = auto_chunks( load, P.max_tile_vol, P.jacc, 0 );
     }
     for ( size_t r = 0; r < sims.size(); r++ ) {
         zpic_sim * s = sims[r];

@@ -1948,7 +1948,6 @@ namespace zb {
 // with 128 threads for the FP32 and FP64 tile currents 32x32-cell tiles took 312 and
 // 339 us per step instead of 204 and 211, 64x64 302 instead of 202 with the
 // fixed-point one.
-constexpr double PK_HEAVY = 4096.0;
 struct PkConfig { int threads, per_sm; size_t smem; };
 static size_t pk_smem( int tile_vol, int jacc, int threads ) {
     return (size_t) ( jacc ? 12 : 9 ) * tile_vol * sizeof( float ) + sizeof( PairFactors ) +

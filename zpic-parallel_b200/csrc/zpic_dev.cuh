@@ -214,6 +214,8 @@ __device__ __forceinline__ int cell_y( uint32_t c ) { return static_cast<int>( s
 
 // Work item of the particle kernels: species, tile, chunk
 struct Item { int sp; int tile; int chunk; int pad; };
+// Particles of a work item from which on its CTA has 256 threads at least.
+constexpr double PK_HEAVY = 4096.0;
 
 // Tiles [tile, tile + SEG_TILES) of a species: work item of the sort's check.
 constexpr int SEG_TILES = 1024;
