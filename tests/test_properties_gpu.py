@@ -88,6 +88,36 @@ def test_relocation_and_repack_free_streaming(capacity):
         assert g.repacks(0) > 0
 
 
+@pytest.mark.parametrize('ntiles', [(41, 27), (64, 33)])
+@pytest.mark.parametrize('capacity', [None, 0.11])
+def test_relocation_and_repack_across_segments(ntiles, capacity):
+    """The same for 1,107 and 2,112 tiles: the sort's check takes 1,024 tiles per CTA, and the CTA that finishes a
+    species' last segment (a ragged one) plans all of them.  The slab crosses every row of tiles, so that tiles of
+    the first and of the last segment overflow."""
+    geom = (ntiles, (8, 8), (0.8 * ntiles[0], 0.8 * ntiles[1]), 0.07)
+
+    def setup(s):
+        s.add_species(-1.0, (4, 4), density=('slab', 1.0, 0.5, 3.0, 0),
+                      udist=('thermal', (0.05, 0.05, 0.05), (0.9, 0.0, 0.0)))
+        return s
+    o = setup(OracleSim(*geom))
+    g = zb.Simulation(*geom)
+    if capacity is not None:
+        g.set_option('capacity_factor', capacity)
+    setup(g)
+    occupied0 = set(np.nonzero(o.tiles(0)[0])[0])
+    for n in range(1, 61):
+        o.species_advance_free(0)
+        g.species_advance(0, zb.ADVANCE_FREE)
+        if n % 15 == 0:
+            assert same_multisets(o.particles(0), g.particles(0)), 'step %d' % n
+    new = set(np.nonzero(o.tiles(0)[0])[0]) - occupied0
+    assert min(new) < 1024 and max(new) >= ntiles[0] * ntiles[1] // 1024 * 1024
+    assert g.relocations(0) > 0
+    if capacity is not None:
+        assert g.repacks(0) > 0
+
+
 @pytest.mark.parametrize('ntiles,bc', [
     ((1, 1), (1, 1, 1, 1)), ((2, 1), (1, 1, 1, 1)), ((1, 2), (1, 1, 1, 1)), ((3, 5), (1, 1, 1, 1)),
     ((3, 5), (0, 0, 1, 1)), ((4, 3), (0, 0, 0, 0)), ((4, 3), (1, 1, 0, 0)),
