@@ -17,11 +17,10 @@ def _sim(ntiles, nx):
     return zb.Simulation(ntiles, nx, (ntiles[0] * nx[0] * dx, ntiles[1] * nx[1] * dx), 0.05)
 
 
-# bytes of one grid: 364 * 12 = 4,368 per 16x16 tile; 64 KiB lies between 15 and 16 tiles, 224 KiB (a chunk)
-# between 52 and 53, 448 KiB between 105 and 106, 2 MiB and 12 MiB (all lanes) between 480 and 481, 2,880 and 2,881
-@pytest.mark.parametrize('ntiles', [(1, 1), (5, 3), (4, 4), (52, 1), (53, 1), (15, 7), (53, 2), (12, 10),
-                                    (11, 11), (16, 15), (241, 1), (30, 16), (37, 13), (32, 30), (31, 31), (64, 45), (43, 67),
-                                    (64, 61)])
+# bytes of one grid: 364 * 12 = 4,368 per 16x16 tile; 64 KiB lies between 15 and 16 tiles, 512 KiB (a chunk) between
+# 120 and 121, 1 MiB (two) between 240 and 241, 2 MiB and 12 MiB (all lanes) between 480 and 481, 2,880 and 2,881
+@pytest.mark.parametrize('ntiles', [(1, 1), (5, 3), (4, 4), (12, 10), (11, 11), (16, 15), (241, 1), (30, 16), (37, 13),
+                                    (31, 31), (64, 45), (43, 67), (64, 61)])
 def test_grid_round_trip(ntiles):
     s = _sim(ntiles, (16, 16))
     a = np.random.default_rng(ntiles[0]).random((ntiles[0] * ntiles[1], s.tile_vol, 3), np.float32)
@@ -33,6 +32,17 @@ def test_grid_round_trip(ntiles):
     d = a[:, :361].reshape(ntiles[1], ntiles[0], 19, 19, 3)[:, :, 1:17, 1:17].transpose(0, 2, 1, 3, 4)
     for k in range(3):
         assert np.array_equal(s.grid_gather('E', k), d.reshape(ntiles[1] * 16, ntiles[0] * 16, 3)[..., k])
+
+
+def test_round_trips_past_the_larger_chunks():
+    """The further lanes' chunks grow after 256 MiB of wide copies: 28 MB at a time, 14 times."""
+    s = _sim((80, 80), (16, 16))
+    a = np.random.default_rng(2).random((6400, s.tile_vol, 3), np.float32)
+    s.set_grid('E', a)
+    s.set_grid('B', -a)
+    for _ in range(7):
+        assert np.array_equal(s.grid('E'), a)
+        assert np.array_equal(s.grid('B'), -a)
 
 
 def test_pinned_destination():

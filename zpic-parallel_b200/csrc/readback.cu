@@ -24,7 +24,9 @@ namespace zb {
 namespace {
 
 constexpr int LANES = 4;
-constexpr size_t CHUNK = 224 * 1024;          // pinned bytes per slot (two slots per lane: all lanes within 2 MB)
+constexpr size_t CHUNK = 512 * 1024;          // pinned bytes per slot (two slots per lane)
+constexpr size_t CHUNK_FIRST = 160 * 1024;    // those of the further lanes until they have copied PAYS bytes
+constexpr size_t PAYS = 256 << 20;
 constexpr size_t SMALL = 64 * 1024;           // the driver's own path is as good below
 // All lanes into fresh pages, and into pages that are there, from this many bytes
 // on, one below.  Waking a thread costs up to 0.25 ms.  With one lane, four lanes
@@ -38,33 +40,41 @@ struct Lane {
     cudaStream_t st = nullptr;                // none for the first lane: it copies on the caller's stream
     cudaEvent_t done[2] = { nullptr, nullptr };
     char * buf = nullptr;                     // two chunks
+    size_t chunk = 0;
 };
 
 // The lanes of one device, made when they are first used and given back when the
 // device's last simulation is destroyed.  The first read-out of a simulation
 // pays for them, so they are made to cost little: the first lane needs no stream,
 // and the driver cuts pinned buffers from blocks of 2 MB, 1.3 ms each, of which
-// every simulation holds one for its scratch: the lanes' 1.75 MB fit the rest of
+// every simulation holds one for its scratch: the lanes' 1.94 MB fit the rest of
 // it (4 MB of buffers and four streams made at once took 2.1 to 5 ms, and 0.9 ms
-// when they were given back; now 0.01 ms, and 0.2 for the three streams of a wide copy).
+// when they were given back; now 0.01 ms, and 0.2 for the three streams of a wide
+// copy).  Small chunks cost a wide copy a tenth, so that after PAYS bytes, 25 ms of
+// copying, the further lanes get large ones as well.
 struct Pool {
     std::mutex busy;
     Lane lane[LANES];
     cudaEvent_t ready = nullptr;
     int made = 0;
+    size_t wide_bytes = 0;
     int users = 0;
 
     // lanes [0, n) are there, or as many as could be made
     void make( int n ) {
         cudaError_t e = cudaSuccess;
         if ( !ready && n > 1 ) e = cudaEventCreateWithFlags( &ready, cudaEventDisableTiming );
-        while ( made < n && e == cudaSuccess ) {
-            Lane & l = lane[made];
-            if ( made > 0 ) e = cudaStreamCreateWithFlags( &l.st, cudaStreamNonBlocking );
-            for ( int k = 0; k < 2; k++ )
-                if ( e == cudaSuccess ) e = cudaEventCreateWithFlags( &l.done[k], cudaEventDisableTiming );
-            if ( e == cudaSuccess ) e = cudaHostAlloc( (void **) &l.buf, 2 * CHUNK, cudaHostAllocPortable );
-            if ( e == cudaSuccess ) made++; else free_lane( l );
+        for ( int k = 0; k < n && e == cudaSuccess; k++ ) {
+            Lane & l = lane[k];
+            const size_t chunk = k == 0 || wide_bytes >= PAYS ? CHUNK : CHUNK_FIRST;
+            if ( l.chunk == chunk ) continue;
+            if ( l.buf ) { cudaFreeHost( l.buf ); l.buf = nullptr; }        // (larger chunks)
+            if ( k > 0 && !l.st ) e = cudaStreamCreateWithFlags( &l.st, cudaStreamNonBlocking );
+            for ( int i = 0; i < 2; i++ )
+                if ( e == cudaSuccess && !l.done[i] ) e = cudaEventCreateWithFlags( &l.done[i], cudaEventDisableTiming );
+            if ( e == cudaSuccess ) e = cudaHostAlloc( (void **) &l.buf, 2 * chunk, cudaHostAllocPortable );
+            if ( e == cudaSuccess ) { l.chunk = chunk; made = std::max( made, k + 1 ); }
+            else { free_lane( l ); made = std::min( made, k ); }
         }
         if ( e != cudaSuccess ) cudaGetLastError();
     }
@@ -79,6 +89,7 @@ struct Pool {
         if ( ready ) cudaEventDestroy( ready );
         ready = nullptr;
         made = 0;
+        wide_bytes = 0;
     }
 };
 
@@ -89,20 +100,20 @@ std::map<int, std::unique_ptr<Pool>> g_pools;
 cudaError_t run_lane( int device, Lane & l, cudaStream_t st, char * dst, const char * src, size_t bytes ) {
     cudaError_t e = cudaSetDevice( device );
     if ( e != cudaSuccess ) return e;
-    const size_t n = ( bytes + CHUNK - 1 ) / CHUNK;
+    const size_t n = ( bytes + l.chunk - 1 ) / l.chunk;
     for ( size_t k = 0; k <= n; k++ ) {
         const int b = (int) ( k & 1 );
         if ( k < n ) {
-            const size_t at = k * CHUNK, len = std::min( CHUNK, bytes - at );
-            e = cudaMemcpyAsync( l.buf + b * CHUNK, src + at, len, cudaMemcpyDeviceToHost, st );
+            const size_t at = k * l.chunk, len = std::min( l.chunk, bytes - at );
+            e = cudaMemcpyAsync( l.buf + b * l.chunk, src + at, len, cudaMemcpyDeviceToHost, st );
             if ( e == cudaSuccess ) e = cudaEventRecord( l.done[b], st );
             if ( e != cudaSuccess ) break;
         }
         if ( k > 0 ) {
-            const size_t at = ( k - 1 ) * CHUNK, len = std::min( CHUNK, bytes - at );
+            const size_t at = ( k - 1 ) * l.chunk, len = std::min( l.chunk, bytes - at );
             e = cudaEventSynchronize( l.done[1 - b] );
             if ( e != cudaSuccess ) break;
-            std::memcpy( dst + at, l.buf + ( 1 - b ) * CHUNK, len );
+            std::memcpy( dst + at, l.buf + ( 1 - b ) * l.chunk, len );
         }
     }
     if ( e != cudaSuccess ) cudaStreamSynchronize( st );       // nothing of this copy is left in flight
@@ -162,6 +173,7 @@ cudaError_t copy_to_host( int device, cudaStream_t st, void * dst, const void * 
     if ( !own.owns_lock() ) return copy_plain( st, dst, src, bytes );
     const bool wide = ( bytes >= WIDE || ( bytes >= WIDE_FRESH && fresh_pages( dst, bytes ) ) ) &&
                       std::thread::hardware_concurrency() >= LANES;
+    if ( wide && pool->wide_bytes < PAYS ) pool->wide_bytes += bytes;
     pool->make( wide ? LANES : 1 );
     if ( pool->made == 0 ) return copy_plain( st, dst, src, bytes );
     const int lanes = wide ? pool->made : 1;
