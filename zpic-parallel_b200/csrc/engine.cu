@@ -48,7 +48,7 @@ cudaError_t launch_yee( cudaStream_t, const TileItem *, int, const RunDev *, int
 cudaError_t launch_emf_bc( cudaStream_t, const RunDev *, int, int, int );
 cudaError_t launch_cur_bc( cudaStream_t, const RunDev *, int, int, int );
 cudaError_t launch_kernel3( cudaStream_t, const TileItem *, int, const RunDev *, int, int, float, float, float, int );
-size_t filter_smem_bytes( int, int, int, int );
+size_t filter_smem_bytes( int, int, int, uint64_t );
 cudaError_t launch_filter( cudaStream_t, const TileItem *, int, const RunDev *, int, int, const float *, const float *, size_t );
 cudaError_t launch_shift_left( cudaStream_t, const TileItem *, int, const RunDev *, int );
 cudaError_t launch_field_energy( cudaStream_t, const RunDev *, int, int, double * );
@@ -477,7 +477,7 @@ static int upload_run( zpic_sim * s ) {
     return ZPIC_OK;
 }
 
-static int filter_npass( const zpic_sim * s );
+static uint64_t filter_npass( const zpic_sim * s );
 
 // Build the work lists for a set of simulations (one sim, or a batch).
 static int plan_build( Plan & P, const std::vector<zpic_sim *> & sims, int chunks_override = 0 ) {
@@ -670,21 +670,18 @@ static int run_sort( Plan & P, cudaStream_t st, int use_extra ) {
     return ZPIC_OK;
 }
 
-// The 3-point passes of a run's filter (filter.h:22-86): a v[-1] + b v[0] + a v[+1] each.
-static void filter_passes( const zpic_sim * s, std::vector<float> & a, std::vector<float> & b ) {
-    const unsigned order = s->forder > 0 ? s->forder : 1;
-    a.assign( order, 0.25f ); b.assign( order, 0.5f );
-    if ( s->ftype == ZPIC_FILTER_COMPENSATED ) {
-        const float ca = -1.0f;
-        const float cb = ( 4.0 + 2.0 * order ) / order;
-        const float norm = 2 * ca + cb;
-        a.push_back( ca / norm ); b.push_back( cb / norm );
-    }
+// Passes of a run's filter (the order is the caller's, any number), and one of
+// them (filter.h:22-86): a v[-1] + b v[0] + a v[+1].
+static uint64_t filter_npass( const zpic_sim * s ) {
+    return s->ftype == ZPIC_FILTER_NONE ? 0 : (uint64_t) s->forder + ( s->ftype == ZPIC_FILTER_COMPENSATED );
 }
-
-// Passes of the filter, capped (the order is the caller's, any number).
-static int filter_npass( const zpic_sim * s ) {
-    return s->ftype == ZPIC_FILTER_NONE ? 0 : (int) std::min<unsigned>( s->forder, 1000 ) + ( s->ftype == ZPIC_FILTER_COMPENSATED );
+static void filter_pass( const zpic_sim * s, uint64_t pass, float & a, float & b ) {
+    a = 0.25f; b = 0.5f;
+    if ( pass < s->forder ) return;
+    const float ca = -1.0f;
+    const float cb = ( 4.0 + 2.0 * s->forder ) / s->forder;
+    const float norm = 2 * ca + cb;
+    a = ca / norm; b = cb / norm;
 }
 
 // Current::advance device part for every run of the plan (current.cpp:227-246).
@@ -716,17 +713,20 @@ static int run_current( Plan & P, cudaStream_t st, bool in_step = false ) {
         const int nt = s->ntx * s->nty;
         first += nt;
         if ( s->ftype == ZPIC_FILTER_NONE ) continue;
-        std::vector<float> a, b;
-        filter_passes( s, a, b );
+        const uint64_t n = filter_npass( s );
         if ( in_step && P.filter_in_one ) {
+            float a[FILTER_PASSES], b[FILTER_PASSES];
+            for ( uint64_t i = 0; i < n; i++ ) filter_pass( s, i, a[i], b[i] );
             PhaseScope ps( prof_sim( P ), st, PH_CURRENT, 1 );
-            DEV( launch_filter( st, items, nt, P.runs_d, s->fdir, (int) a.size(), a.data(), b.data(),
-                                filter_smem_bytes( s->run.extx, s->run.exty, s->fdir, (int) a.size() ) ) );
+            DEV( launch_filter( st, items, nt, P.runs_d, s->fdir, (int) n, a, b,
+                                filter_smem_bytes( s->run.extx, s->run.exty, s->fdir, n ) ) );
             continue;
         }
-        for ( size_t i = 0; i < a.size(); i++ ) {
+        for ( uint64_t i = 0; i < n; i++ ) {
+            float a, b;
+            filter_pass( s, i, a, b );
             PhaseScope ps( prof_sim( P ), st, PH_CURRENT, 2 );
-            DEV( launch_kernel3( st, items, nt, P.runs_d, 2, s->fdir, a[i], b[i], a[i], P.max_tile_vol ) );
+            DEV( launch_kernel3( st, items, nt, P.runs_d, 2, s->fdir, a, b, a, P.max_tile_vol ) );
             DEV( launch_cur_gc( st, items, nt, P.runs_d, s->fdir ? 2 : 1, P.max_guard ) );
         }
     }

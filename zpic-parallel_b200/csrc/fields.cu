@@ -645,7 +645,7 @@ k_kernel3( const TileItem * __restrict__ items, const RunDev * __restrict__ runs
 // no neighbour the guard cells are constants, as there.  The passes one by one
 // took two kernels each of 5 us on a small grid (256x64, three passes: 31 us),
 // a chain that the step waited for.
-constexpr int FILTER_THREADS = 256, FILTER_PASSES = 8;
+constexpr int FILTER_THREADS = 256;
 struct FilterSpec { int diry, npass; float a[FILTER_PASSES], b[FILTER_PASSES]; };      // a v[-1] + b v[0] + a v[+1]
 
 __global__ void __launch_bounds__( FILTER_THREADS )
@@ -876,10 +876,10 @@ cudaError_t launch_kernel3( cudaStream_t st, const TileItem * items, int n, cons
 }
 // Shared memory of k_filter for tiles of extx x exty cells, 0 when it cannot
 // take them: the passes must stay within the neighbours' interiors.
-size_t filter_smem_bytes( int extx, int exty, int diry, int npass ) {
+size_t filter_smem_bytes( int extx, int exty, int diry, uint64_t npass ) {
     const int nu = ( diry ? exty : extx ) - GL - GU;
-    if ( npass < 1 || npass > FILTER_PASSES || npass > nu - GU ) return 0;
-    const size_t b = 6 * sizeof( float ) * (size_t) ( ( diry ? exty : extx ) + 2 * npass ) * ( diry ? extx : exty );
+    if ( npass < 1 || npass > (uint64_t) FILTER_PASSES || (int) npass > nu - GU ) return 0;
+    const size_t b = 6 * sizeof( float ) * ( (size_t) ( diry ? exty : extx ) + 2 * npass ) * ( diry ? extx : exty );
     return b <= 200 * 1024 ? b : 0;
 }
 cudaError_t launch_filter( cudaStream_t st, const TileItem * items, int n, const RunDev * runs, int diry, int npass,

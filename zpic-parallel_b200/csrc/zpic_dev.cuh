@@ -217,6 +217,9 @@ struct Item { int sp; int tile; int chunk; int pad; };
 // Particles of a work item from which on its CTA has 256 threads at least.
 constexpr double PK_HEAVY = 4096.0;
 
+// Passes of a current filter that one kernel (k_filter) takes.
+constexpr int FILTER_PASSES = 8;
+
 // Tiles [tile, tile + SEG_TILES) of a species: work item of the sort's check.
 constexpr int SEG_TILES = 1024;
 struct SegItem { int sp; int tile; };
