@@ -183,7 +183,8 @@ int zpic_b200_sim_synchronize( zpic_sim * sim );
  *                         share of their number (default 0.5; at least twice
  *                         the minimum slack of ppc * cells / 8)
  *   "wait_limit"     n    polls before a kernel's bounded wait on its bulk
- *                         copies gives up (default 4194304, ~0.5 s); a kernel
+ *                         copies gives up (default 4194304, 17 s: a poll
+ *                         after the first may take 4 us); a kernel
  *                         that gives up skips its work for that tile and the
  *                         next synchronising call returns ZPIC_E_DEVICE
  */

@@ -1623,7 +1623,7 @@ int zpic_b200_sim_set_option( zpic_sim * s, const char * key, double v ) {
     }
     else if ( k == "wait_limit" ) {
         // polls of the kernels' bounded waits on their bulk copies before
-        // they give up (default ~0.5 s worth)
+        // they give up (default 17 s worth)
         const int w = (int) v;
         if ( w < 1 || w != v ) return fail( ZPIC_E_INVALID, "wait_limit must be a poll count >= 1" );
         s->run.wait_limit = w;

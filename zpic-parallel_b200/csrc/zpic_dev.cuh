@@ -174,7 +174,7 @@ __device__ __forceinline__ void bulk_wait_all() {
     asm volatile( "cp.async.bulk.wait_group 0;" ::: "memory" );
 }
 
-// Polls of a bounded wait by default: ~0.5 s.
+// Polls of a bounded wait by default: 17 s (a poll may take 4.1 us).
 constexpr int WAIT_LIMIT_DEFAULT = 1 << 22;
 
 // Bounded wait on an mbarrier phase.  Gives up after `limit` polls, records
