@@ -1,6 +1,7 @@
-"""The field solve that sums the deposits of the tiles itself, and the current filter in one kernel (whole
-steps), against the separate sum, filter passes and solve (the same step issued object by object): J, E and B, guard cells included, bit for bit.  One species with one
-CTA per tile: its fixed-point deposits do not depend on the order of the sums, so there is no rounding to allow."""
+"""The field solve that sums the deposits of the tiles itself, and the current filter in one kernel (whole steps),
+against the separate sum, filter passes and solve (the same step issued object by object): J, E and B, guard cells
+included, bit for bit.  One species with one CTA per tile: its fixed-point deposits do not depend on the order of
+the sums, so there is no rounding to allow."""
 import numpy as np
 import pytest
 
